@@ -1,93 +1,311 @@
 // True float32 matrix product on the CUDA cores (no tensor-core mode, no reduced precision):
 //   out[T, N] = a[T, K] . w[N, K]^T (+ bias[N])
-// Every output element is accumulated by one thread over k = 0 .. K-1 in ascending order with
-// fused multiply-adds, so the value of a row does not depend on how many other rows are in the
-// batch or on where the row sits in it.
+//
+// One order of additions for every shape of the batch, so that the value of a row does not depend on
+// how many other rows are in the batch, on where the row sits in it, or on which kernel runs:
+//   K is cut into at most 32 slices of SL = 8 ceil(K / 256) elements, and eight slices make a group;
+//   a slice is summed by fused multiply-adds over ascending k from zero, a group is the sum of its
+//   slices in ascending order from zero, and the result the sum of the groups in the same way, + bias.
+// What is cut can be worked on side by side, which is what a step of a few rows needs: as a single
+// chain of K additions per output a product of 6 rows at K = 576 .. 1536 took 66 us on average.
+//
+//   few rows   one block owns NB output features for all of K, a warp lane one slice: meant to be bound by
+//              streaming w once; measured it is the latency of a block (load, multiply, 32 partial sums), with
+//              two blocks of 110 KB per SM. 6 rows, K = 576: 49152 features 64 us (w at copy rate: 17), 3072
+//              features 12 us; 576 features of K = 1536 12 us (all with 6 us of start and timing);
+//   tiles      BM x BN outputs per block, 4 x 4 per thread, the next K tile on its way in registers
+//              while this one is multiplied: bound by the FMA units. Where 64 x 64 tiles would leave
+//              SMs idle, 32 x 32 tiles whose four groups of K are summed by four sets of threads.
 #include "common.cuh"
 #include "kernels.h"
 
 namespace lse {
+namespace gf32 {
 
-constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;  // 256 threads, 4x4 outputs each
+constexpr int SLICES = 32, GROUP = 8;
 
-__global__ void __launch_bounds__(256)
-gemm_f32_kernel(const float* __restrict__ a, const float* __restrict__ w,
-                const float* __restrict__ bias, float* __restrict__ out, int T, int N, int K) {
-  __shared__ float as[BK][BM + 4];
-  __shared__ float ws[BK][BN + 4];
-  const int tid = threadIdx.x;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  const int tm = (tid / 16) * TM, tn = (tid % 16) * TN;
-  float acc[TM][TN];
-#pragma unroll
-  for (int i = 0; i < TM; ++i)
-#pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+__host__ __device__ inline int slice_len(int K) { return (K + SLICES * 8 - 1) / (SLICES * 8) * 8; }
 
-  // each thread loads 4 consecutive k of one row of each tile
-  const int lr = tid / 4, lk = (tid % 4) * 4;
-  const bool vec_ok = (K % 4 == 0);
-  for (int k0 = 0; k0 < K; k0 += BK) {
-    float av[4] = {0.f, 0.f, 0.f, 0.f}, wv[4] = {0.f, 0.f, 0.f, 0.f};
-    const int gm = m0 + lr, gn = n0 + lr, gk = k0 + lk;
-    if (gm < T) {
-      if (vec_ok && gk + 3 < K) {
-        const float4 v = *reinterpret_cast<const float4*>(a + (size_t)gm * K + gk);
-        av[0] = v.x; av[1] = v.y; av[2] = v.z; av[3] = v.w;
-      } else {
+struct Args {
+  const float* a;
+  const float* w;
+  const float* bias;
+  float* out;
+  int T, N, K, SL;
+};
+
+// ---------------------------------------------------------------------------------------- few rows
+// NG warps, each NPT features of w and 8 rows of a; lane s sums slice s. A pass brings 8 elements of every
+// slice of every row. A staged slice is 12 floats apart from the next: eight neighbouring lanes then read
+// 16 bytes each from 8 different groups of banks.
+constexpr int FEW_T = 8, CH = 8, PAD = 12, ROW = SLICES * PAD, STAGES = 3;
+
+__device__ __forceinline__ void copy16(float* smem, const float* gmem, bool valid) {
+  const uint32_t dst = (uint32_t)__cvta_generic_to_shared(smem);
+  const int bytes = valid ? 16 : 0;  // the rest is filled with zeros
+  asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(gmem), "r"(bytes));
+}
+
+template <int NPT, int NG>
+__global__ void __launch_bounds__(32 * NG) few_rows_kernel(const Args p) {
+  constexpr int NB = NPT * NG, THREADS = 32 * NG;
+  extern __shared__ __align__(16) float smem[];
+  pdl_trigger();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int n0 = blockIdx.x * NB, t0 = blockIdx.y * FEW_T;
+  const int passes = p.SL / CH;
+  auto load = [&](int c, int rows, int first, const float* src, int r0, int limit) {
+    float* buf = smem + (c % STAGES) * (NB + FEW_T) * ROW + first * ROW;
+    for (int i = threadIdx.x; i < rows * SLICES * 2; i += THREADS) {
+      const int half = i & 1, s = (i >> 1) & (SLICES - 1), r = i / (SLICES * 2);
+      const int k = s * p.SL + c * CH + half * 4;
+      const bool valid = k < p.K && r0 + r < limit;  // K is a multiple of 4 here
+      copy16(buf + r * ROW + s * PAD + half * 4, valid ? src + (size_t)(r0 + r) * p.K + k : src, valid);
+    }
+  };
+  // the weights depend on no earlier kernel: the first passes' are asked for before the wait
+  for (int c = 0; c < STAGES - 1 && c < passes; ++c) load(c, NB, 0, p.w, n0, p.N);
+  pdl_wait();
+  for (int c = 0; c < STAGES - 1; ++c) {
+    if (c < passes) load(c, FEW_T, NB, p.a, t0, p.T);
+    asm volatile("cp.async.commit_group;\n" ::);
+  }
+  float acc[FEW_T][NPT];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) if (gk + j < K) av[j] = a[(size_t)gm * K + gk + j];
+  for (int t = 0; t < FEW_T; ++t)
+#pragma unroll
+    for (int j = 0; j < NPT; ++j) acc[t][j] = 0.f;
+  for (int c = 0; c < passes; ++c) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(STAGES - 2));
+    __syncthreads();  // pass c is there, and everybody is done with the buffer that is filled next
+    if (c + STAGES - 1 < passes) {
+      load(c + STAGES - 1, NB, 0, p.w, n0, p.N);
+      load(c + STAGES - 1, FEW_T, NB, p.a, t0, p.T);
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
+    const float* buf = smem + (c % STAGES) * (NB + FEW_T) * ROW + lane * PAD;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      float4 wv[NPT];
+#pragma unroll
+      for (int j = 0; j < NPT; ++j)
+        wv[j] = *reinterpret_cast<const float4*>(buf + (warp * NPT + j) * ROW + half * 4);
+#pragma unroll
+      for (int t = 0; t < FEW_T; ++t) {
+        const float4 av = *reinterpret_cast<const float4*>(buf + (NB + t) * ROW + half * 4);
+#pragma unroll
+        for (int j = 0; j < NPT; ++j) {
+          acc[t][j] = fmaf(av.x, wv[j].x, acc[t][j]);
+          acc[t][j] = fmaf(av.y, wv[j].y, acc[t][j]);
+          acc[t][j] = fmaf(av.z, wv[j].z, acc[t][j]);
+          acc[t][j] = fmaf(av.w, wv[j].w, acc[t][j]);
+        }
       }
-    }
-    if (gn < N) {
-      if (vec_ok && gk + 3 < K) {
-        const float4 v = *reinterpret_cast<const float4*>(w + (size_t)gn * K + gk);
-        wv[0] = v.x; wv[1] = v.y; wv[2] = v.z; wv[3] = v.w;
-      } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) if (gk + j < K) wv[j] = w[(size_t)gn * K + gk + j];
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      as[lk + j][lr] = av[j];
-      ws[lk + j][lr] = wv[j];
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < BK; ++kk) {
-      float ar[TM], wr[TN];
-#pragma unroll
-      for (int i = 0; i < TM; ++i) ar[i] = as[kk][tm + i];
-#pragma unroll
-      for (int j = 0; j < TN; ++j) wr[j] = ws[kk][tn + j];
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(ar[i], wr[j], acc[i][j]);
     }
   }
+  asm volatile("cp.async.wait_group 0;\n" ::);
+  __syncthreads();
+  float* red = smem;  // [FEW_T * NB][SLICES + 1]
 #pragma unroll
-  for (int i = 0; i < TM; ++i) {
-    const int gm = m0 + tm + i;
-    if (gm >= T) continue;
+  for (int t = 0; t < FEW_T; ++t)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) {
-      const int gn = n0 + tn + j;
-      if (gn < N) out[(size_t)gm * N + gn] = acc[i][j] + (bias ? bias[gn] : 0.f);
+    for (int j = 0; j < NPT; ++j) red[(t * NB + warp * NPT + j) * (SLICES + 1) + lane] = acc[t][j];
+  __syncthreads();
+  for (int o = threadIdx.x; o < FEW_T * NB; o += THREADS) {
+    const int t = t0 + o / NB, n = n0 + o % NB;
+    const float* r = red + o * (SLICES + 1);
+    float total = 0.f;
+#pragma unroll
+    for (int g = 0; g < SLICES / GROUP; ++g) {
+      float sum = 0.f;
+#pragma unroll
+      for (int s = 0; s < GROUP; ++s) sum += r[g * GROUP + s];
+      total += sum;
+    }
+    if (t < p.T && n < p.N) p.out[(size_t)t * p.N + n] = total + (p.bias ? p.bias[n] : 0.f);
+  }
+}
+
+// ---------------------------------------------------------------------------------------- tiles
+// G sets of threads; set g sums the groups of slices g * 4 / G .. of K (G = 1: all of them).
+constexpr int BK = 16;
+
+template <int BM, int BN, int G>
+__global__ void __launch_bounds__(G * (BM / 4) * (BN / 4)) tiles_kernel(const Args p, const bool vec) {
+  constexpr int SET = (BM / 4) * (BN / 4);              // threads of a set
+  constexpr int PA = BM * 4 / SET, PW = BN * 4 / SET;   // pieces of four k per thread and tile
+  static_assert(BM * 4 % SET == 0 && BN * 4 % SET == 0, "");
+  constexpr int LA = BM + 4, LW = BN + 4, TILE = BK * (LA + LW);
+  __shared__ __align__(16) float smem[G * 2 * TILE];
+  static_assert(G == 1 || G * BM * BN <= G * 2 * TILE, "");
+  pdl_trigger();
+  const int set = threadIdx.x / SET, tid = threadIdx.x % SET;
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  const int tm = (tid / (BN / 4)) * 4, tn = (tid % (BN / 4)) * 4;
+  float* tiles = smem + set * 2 * TILE;
+  const int per_set = SLICES / G * p.SL;                // elements of K per set, a multiple of BK
+  const int k_begin = set * per_set;
+  const int n_tiles = ((G == 1 ? p.K : min(p.K, per_set)) + BK - 1) / BK;  // the same for every set
+  float acc[4][4], grp[4][4], tot[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = grp[i][j] = tot[i][j] = 0.f;
+  float4 av[PA], wv[PW];
+  auto piece = [&](const float* src, int row, int limit, int k) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (row < limit) {
+      const float* q = src + (size_t)row * p.K + k;
+      if (vec) {
+        if (k < p.K) v = *reinterpret_cast<const float4*>(q);
+      } else {
+        if (k < p.K) v.x = q[0];
+        if (k + 1 < p.K) v.y = q[1];
+        if (k + 2 < p.K) v.z = q[2];
+        if (k + 3 < p.K) v.w = q[3];
+      }
+    }
+    return v;
+  };
+  auto fetch = [&](int it) {
+    const int k0 = k_begin + it * BK;
+#pragma unroll
+    for (int i = 0; i < PA; ++i) {
+      const int idx = tid + i * SET;
+      av[i] = piece(p.a, m0 + idx / 4, p.T, k0 + idx % 4 * 4);
+    }
+#pragma unroll
+    for (int i = 0; i < PW; ++i) {
+      const int idx = tid + i * SET;
+      wv[i] = piece(p.w, n0 + idx / 4, p.N, k0 + idx % 4 * 4);
+    }
+  };
+  auto put = [&](int buf) {
+    float* as = tiles + buf * TILE;
+    float* ws = as + BK * LA;
+#pragma unroll
+    for (int i = 0; i < PA; ++i) {
+      const int idx = tid + i * SET, r = idx / 4, k = idx % 4 * 4;
+      as[k * LA + r] = av[i].x; as[(k + 1) * LA + r] = av[i].y;
+      as[(k + 2) * LA + r] = av[i].z; as[(k + 3) * LA + r] = av[i].w;
+    }
+#pragma unroll
+    for (int i = 0; i < PW; ++i) {
+      const int idx = tid + i * SET, r = idx / 4, k = idx % 4 * 4;
+      ws[k * LW + r] = wv[i].x; ws[(k + 1) * LW + r] = wv[i].y;
+      ws[(k + 2) * LW + r] = wv[i].z; ws[(k + 3) * LW + r] = wv[i].w;
+    }
+  };
+  auto add_into = [](float (&to)[4][4], float (&from)[4][4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        to[i][j] += from[i][j];
+        from[i][j] = 0.f;
+      }
+  };
+  pdl_wait();
+  fetch(0);
+  put(0);
+  __syncthreads();
+  int left = p.SL, slices = GROUP;
+  for (int it = 0; it < n_tiles; ++it) {
+    if (it + 1 < n_tiles) fetch(it + 1);
+    const float* as = tiles + (it & 1) * TILE + tm;
+    const float* ws = tiles + (it & 1) * TILE + BK * LA + tn;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+#pragma unroll
+      for (int kk = 8 * half; kk < 8 * half + 8; ++kk) {
+        const float4 x = *reinterpret_cast<const float4*>(as + kk * LA);
+        const float4 y = *reinterpret_cast<const float4*>(ws + kk * LW);
+        const float xr[4] = {x.x, x.y, x.z, x.w}, yr[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(xr[i], yr[j], acc[i][j]);
+      }
+      left -= 8;
+      if (left == 0) {  // the end of a slice
+        left = p.SL;
+        add_into(grp, acc);
+        if (--slices == 0) {
+          slices = GROUP;
+          if (G == 1) add_into(tot, grp);
+        }
+      }
+    }
+    if (it + 1 < n_tiles) put((it + 1) & 1);
+    __syncthreads();
+  }
+  add_into(grp, acc);  // what is left of the last slice (zeros after a whole one)
+  add_into(tot, grp);
+  if constexpr (G > 1) {  // the sets' sums meet in shared memory, in order
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      *reinterpret_cast<float4*>(smem + (set * BM + tm + i) * BN + tn) =
+          make_float4(tot[i][0], tot[i][1], tot[i][2], tot[i][3]);
+    __syncthreads();
+    for (int o = threadIdx.x; o < BM * BN; o += G * SET) {
+      const int m = m0 + o / BN, n = n0 + o % BN;
+      float total = 0.f;
+#pragma unroll
+      for (int g = 0; g < G; ++g) total += smem[g * BM * BN + o];
+      if (m < p.T && n < p.N) p.out[(size_t)m * p.N + n] = total + (p.bias ? p.bias[n] : 0.f);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int m = m0 + tm + i;
+      if (m >= p.T) continue;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int n = n0 + tn + j;
+        if (n < p.N) p.out[(size_t)m * p.N + n] = tot[i][j] + (p.bias ? p.bias[n] : 0.f);
+      }
     }
   }
 }
 
+template <int NPT, int NG>
+static cudaError_t launch_few(const Args& p, cudaStream_t stream) {
+  constexpr int NB = NPT * NG, smem = STAGES * (NB + FEW_T) * ROW * 4;
+  static_assert(FEW_T * NB * (SLICES + 1) * 4 <= smem, "");
+  static const cudaError_t configured =
+      cudaFuncSetAttribute(few_rows_kernel<NPT, NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (configured != cudaSuccess) return configured;
+  const dim3 grid((p.N + NB - 1) / NB, (p.T + FEW_T - 1) / FEW_T);
+  return lse::launch(few_rows_kernel<NPT, NG>, grid, 32 * NG, smem, stream, p);
+}
+
+template <int BM, int BN, int G>
+static cudaError_t launch_tiles(const Args& p, bool vec, cudaStream_t stream) {
+  const dim3 grid((p.N + BN - 1) / BN, (p.T + BM - 1) / BM);
+  if (grid.y > 65535) return cudaErrorInvalidValue;
+  return lse::launch(tiles_kernel<BM, BN, G>, grid, G * (BM / 4) * (BN / 4), 0, stream, p, vec);
+}
+
+}  // namespace gf32
 }  // namespace lse
 
 extern "C" int lse_gemm_f32(const float* a, const float* w, const float* bias, float* out, int T,
                             int N, int K, cudaStream_t stream) {
+  using namespace lse::gf32;
   if (T <= 0 || N <= 0) return LSE_OK;
-  if (K <= 0) return LSE_BAD_ARGUMENT;
-  dim3 grid((N + lse::BN - 1) / lse::BN, (T + lse::BM - 1) / lse::BM);
-  if (grid.y > 65535) return LSE_BAD_ARGUMENT;
-  lse::gemm_f32_kernel<<<grid, 256, 0, stream>>>(a, w, bias, out, T, N, K);
-  return cudaPeekAtLastError() == cudaSuccess ? LSE_OK : LSE_LAUNCH_FAILED;
+  if (K <= 0 || (T + 63) / 64 > 65535) return LSE_BAD_ARGUMENT;
+  const Args p{a, w, bias, out, T, N, K, slice_len(K)};
+  const bool vec = K % 4 == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
+  // Measured alone with w out of L2, few rows / tiles in us (each with 6 us of start and timing), N x K, before /
+  // with more rows: 960 x 576 10 / 18 at 16 rows, 16 / 18 at 64; 3072 x 576 16 / 20 at 16, 33 / 27 at 64;
+  // 2048 x 2048 22 / 41 at 16, 35 / 41 at 32, 49 / 41 at 48; 16384 x 2048 72 / 96 at 8, 115 / 98 at 16, 166 / 100 at
+  // 24; 49152 x 576 64 / 137 at 8, 111 / 137 at 16, 174 / 137 at 24. A pass of 8 rows costs as much as the first
+  // one where w is large, almost nothing where the blocks are too few to fill the SMs.
+  const bool few = vec && (T <= 16 || (T <= 32 && N <= 4096));
+  // 64 x 64 tiles once they give every SM two blocks (900 rows, 3072 x 576: 125 us, 26 TFLOP/s); below that 32 x 32
+  const bool wide = (long long)((T + 63) / 64) * ((N + 63) / 64) >= 2 * 148 || (T + 31) / 32 > 65535;
+  const cudaError_t e = few    ? launch_few<4, 4>(p, stream)
+                        : wide ? launch_tiles<64, 64, 1>(p, vec, stream)
+                               : launch_tiles<32, 32, 4>(p, vec, stream);
+  return e == cudaSuccess ? LSE_OK : LSE_LAUNCH_FAILED;
 }

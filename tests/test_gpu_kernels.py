@@ -84,6 +84,22 @@ def test_gemm_f32_is_true_float32_and_batch_invariant(ops, T, N, K, bias):
     assert torch.equal(alone[0], got[T // 2])
 
 
+@pytest.mark.parametrize("N,K", [(1, 4), (16, 256), (17, 260), (576, 1536), (4097, 72), (130, 1001), (9500, 40)])
+def test_gemm_f32_every_kernel_adds_in_the_same_order(ops, N, K):
+    """Few rows, small tiles and large tiles: every row has the same bits from each, and lies within the error of
+    a chain of additions as long as a slice, a group, the groups and the bias together."""
+    w, b = rnd(N, K, seed=2), rnd(N, seed=3)
+    a = rnd(320, K, seed=1)
+    run = lambda rows: ops.linear(rows.clone().cuda(), w.cuda(), b.cuda(), out_dtype=torch.float32).cpu()
+    whole = run(a)
+    ref = a.double() @ w.double().T + b.double()
+    size = a.double().abs() @ w.double().abs().T + b.double().abs()
+    chain = -(-K // 256) * 8 + 8 + 4 + 1
+    assert ((whole.double() - ref).abs() <= 1.01 * chain * 2.0**-24 * size).all()
+    for first, n in ((0, 1), (3, 8), (5, 9), (7, 16), (9, 17), (100, 32), (200, 33), (255, 65)):
+        assert torch.equal(run(a[first : first + n]), whole[first : first + n]), (first, n)
+
+
 @pytest.mark.parametrize("T,N,K", [(1, 48, 64), (9, 520, 200), (16, 128, 64), (17, 2048, 2048),
                                    (8, 16384, 2048), (4, 49152, 2048), (8, 6144, 2048), (2, 2048, 8192),
                                    (64, 136, 1000), (100, 384, 8192), (256, 1000, 520), (300, 136, 1000)])
