@@ -5,22 +5,26 @@
 //   S = Q K^T        tcgen05.mma, A = Q tile and B = K tile in shared memory (both K-major, TMA with
 //                    128-byte swizzle, K tiles fetched page by page through the block table),
 //                    accumulator S [128 x 64] float32 in tensor memory;
-//   softmax          256 threads, two per query row: the keys of every tile are dealt to two
-//                    *streams* (keys 0-31 and 32-63 of the tile), and each stream is a complete
-//                    online softmax of its own: tcgen05.ld of its 32 scores, running maximum and sum
-//                    in float32 (base-2 exponent, scale folded into the multiply-add), P rounded to
-//                    bfloat16 and written back to tensor memory with tcgen05.st. The two threads of
-//                    a row never talk to each other until the end, so twice as many independent
-//                    instruction chains hide the latencies of tensor memory and of the exp unit;
-//   O_s += P_s V_s   per stream s: tcgen05.mma with A = P from tensor memory and B = the stream's 32
-//                    rows of the V tile in shared memory (N-major: rows are keys), accumulator
-//                    O_s [128 x 64] float32 in tensor memory;
+//   softmax          256 threads, two per query row: even tiles are *stream* 0, odd tiles stream 1, and each
+//                    stream is a complete online softmax of its own: tcgen05.ld of its 64 scores, running
+//                    maximum and sum in float32 (base-2 exponent, scale folded into the multiply-add), P
+//                    rounded to bfloat16 and written back to tensor memory with tcgen05.st. The two threads of
+//                    a row never talk to each other until the end;
+//   O_s += P_s V     per stream s: tcgen05.mma with A = P from tensor memory and B = the V tile in shared
+//                    memory (N-major: rows are keys), accumulator O_s [128 x 64] float32 in tensor memory;
 //   end              O = (O_0 w_0 + O_1 w_1) / (l_0 w_0 + l_1 w_1), w_s = 2^(m_s - max m): each thread
 //                    of a row writes half of the head dims.
 // A stream's reference maximum moves only when a row of the warp outgrows it by 2^8; only then is
 // its O rescaled in tensor memory (tcgen05.ld / st) before its next P V. Warps 0-3 are stream 0 and warps 4-7
 // stream 1 (warp w owns tensor-memory lanes 32 (w mod 4) ..), one lane of warp 8 runs the TMA
 // pipeline, one lane of warp 9 issues the MMAs. Every barrier wait is bounded.
+//
+// What bounds it: the exp unit (16 per clock and SM) and, short of that, the latencies of a tile: wait, tcgen05.ld,
+// maximum, exponentials, tcgen05.st, arrival, P V, next Q K^T. A thread therefore takes 64 scores per round, the
+// two streams of a block are never in step, and two blocks share an SM. Pages of 16 tokens make eight copies per
+// tile; issued by one lane they were what a tile waited for. 2040 rows behind 6144 keys, 9 heads: 123 us (one lane
+// issuing, both streams on halves of one tile) -> 94 us -> 60 us with the keys shared by two blocks (exp unit alone:
+// 29 us); 2048 rows behind 4096 keys, 32 heads: 166 -> 141 us (75 us); 2048 rows alone, 32 heads: 45 -> 47 us (15 us).
 #pragma once
 
 #include "attention_args.h"
@@ -34,14 +38,13 @@ using namespace tma;
 constexpr int HD = 64;           // head size served by this kernel
 constexpr int QT = 128;          // query rows per block
 constexpr int KT = 64;           // keys per tile
-constexpr int STAGES = 3;        // key/value tiles in flight
+constexpr int STAGES = 4;        // key/value tiles in flight
 constexpr int SOFTMAX_WARPS = 8;  // two streams of four warps
 constexpr int THREADS = (SOFTMAX_WARPS + 2) * 32;
 constexpr uint32_t Q_BYTES = QT * HD * 2, KV_BYTES = KT * HD * 2;
-// Tensor-memory columns. S is double-buffered so that Q K^T of the next tile runs while the
-// softmax threads work on this one. A stream's P (16 packed columns) is written over the start of
-// that stream's own 32 columns of the S buffer once they are in registers; MMAs of one thread run
-// in issue order, so a later Q K^T into that buffer cannot overtake the P V that still reads P.
+// Tensor-memory columns: S and O of each stream. A stream's P (32 packed columns) is written over its own S once
+// that is in registers; MMAs of one thread run in issue order, so the stream's next Q K^T cannot overtake the
+// P V that still reads P.
 constexpr uint32_t COL_S = 0, S_COLS = 64, COL_O = 128, O_COLS = 64, TMEM_COLS = 256;
 
 __device__ __forceinline__ void umma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
@@ -105,6 +108,44 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// Two float32 operations in one instruction; both halves are rounded as fmaf and + round.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, z, w;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+      "fma.rn.f32x2 w, x, y, z;\n\tmov.b64 {%0, %1}, w;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, w;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+      "add.rn.f32x2 w, x, y;\n\tmov.b64 {%0, %1}, w;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// This block's shared-memory address `addr` in block `rank` of the cluster.
+__device__ __forceinline__ uint32_t peer_address(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void store_peer4(uint32_t addr, float a, float b, float c, float d) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+__device__ __forceinline__ void store_peer2(uint32_t addr, float a, float b) {
+  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(a), "f"(b) : "memory");
+}
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
@@ -117,8 +158,16 @@ struct Params {
   int* error_flag;
 };
 
-// CAP: the scores are scaled and soft-capped as they leave tensor memory.
-template <bool CAP>
+// A cluster of `parts` blocks (1, 2 or 4) shares the keys of one (query tile, head); at the end every block
+// merges 64 / parts head dims of all rows. Its inbox, where the key and value tiles were: [part][row][64 / parts + 4]
+// sums, then [part][row] (maximum, sum).
+__host__ __device__ constexpr int inbox_row(int parts) { return HD / parts + 4; }
+__host__ __device__ constexpr int inbox_bytes(int parts) {
+  return parts > 1 ? parts * QT * (inbox_row(parts) + 2) * 4 : 0;
+}
+
+// CAP: the scores are scaled and soft-capped as they leave tensor memory. PARTS: blocks per (query tile, head).
+template <bool CAP, int PARTS>
 __global__ void __launch_bounds__(THREADS, 2)
 prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                   const __grid_constant__ CUtensorMap map_v, const Params p) {
@@ -132,11 +181,12 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   uint64_t* q_full = bars;                 // [1]
   uint64_t* kv_full = bars + 1;            // [STAGES]
   uint64_t* kv_empty = kv_full + STAGES;   // [STAGES]
-  uint64_t* s_full = kv_empty + STAGES;    // [2] S of a tile is in tensor memory (buffer tile & 1)
-  uint64_t* p_full = s_full + 2;           // [stream][tile & 1] the stream's P is written (and its O
-                                           // rescaled): 4 arrivals
-  uint64_t* pv_done = p_full + 4;          // [2] O_s += P_s V_s of this tile has finished
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 2);
+  uint64_t* s_full = kv_empty + STAGES;    // [stream] S of the stream's next tile is in tensor memory
+  uint64_t* p_full = s_full + 2;           // [stream] its P is written (and its O rescaled): 4 arrivals
+  uint64_t* o_done = p_full + 2;           // [1] every P V has finished
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 1);
+  float* inbox = reinterpret_cast<float*>(k_tiles);
+  static_assert(inbox_bytes(PARTS) <= 2 * STAGES * (int)KV_BYTES, "");
   __shared__ float pair_m[2][QT], pair_l[2][QT];  // the streams' final maxima and sums
   __shared__ volatile int failed;
   __shared__ volatile int issued;  // key/value tiles the producer has requested
@@ -145,7 +195,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // heads vary fastest over the grid, tiles (longest first) slowest: every head's long tiles start early
   const int seq = a.tiles[2 * blockIdx.y], q0 = a.tiles[2 * blockIdx.y + 1];
-  const int head = blockIdx.x;
+  const int head = blockIdx.x / PARTS, part = PARTS > 1 ? (int)cluster_rank() : 0;
   const int kvh = head / (a.num_heads / a.num_kv_heads);
   const int q_start = a.cu_q[seq];
   const int q_len = a.cu_q[seq + 1] - q_start;
@@ -153,7 +203,9 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   const int pos0 = ctx - q_len;
   const int rows_here = min(QT, q_len - q0);
   const int k_end = pos0 + q0 + rows_here;  // one past the last key any row of the tile reads
-  const int n_tiles = (k_end + KT - 1) / KT;
+  const int all_tiles = (k_end + KT - 1) / KT;
+  const int t_first = all_tiles * part / PARTS;              // this block's tiles of keys
+  const int n_tiles = all_tiles * (part + 1) / PARTS - t_first;
 
   if (threadIdx.x == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_q) : "memory");
@@ -168,9 +220,9 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     }
     mbar_init(&s_full[0], 1);
     mbar_init(&s_full[1], 1);
-    for (int b = 0; b < 4; ++b) mbar_init(&p_full[b], 4);
-    mbar_init(&pv_done[0], 1);
-    mbar_init(&pv_done[1], 1);
+    mbar_init(&p_full[0], 4);
+    mbar_init(&p_full[1], 4);
+    mbar_init(o_done, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
@@ -192,8 +244,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   if (warp == SOFTMAX_WARPS) {
     // ---- TMA producer. The whole warp looks up block-table entries, one box of a key/value tile
     // per lane and 32 boxes at a time, so that the lookups of several tiles are one round trip
-    // to memory; lane 0 then waits for free stages and issues the copies, with the rows handed
-    // over by shuffles. The other lanes rest at the warp barrier meanwhile.
+    // to memory; the lanes that hold a tile's rows then issue its copies themselves, keys and values.
     if (lane == 0) {
       mbar_expect_tx(q_full, Q_BYTES);
       tma_load_2d(q_tile, &map_q, q_full, head * HD, q_start + q0);
@@ -202,12 +253,13 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     const int last_page_idx = (k_end - 1) >> p.page_shift;
     const int boxes = KT / p.box_rows;  // 1, 2, 4 or 8
     const int group = 32 / boxes;       // tiles looked up together
+    const int t_mine = lane / boxes, b_l = lane % boxes;
     int ok = 1;
     for (int g0 = 0; g0 < n_tiles && ok; g0 += group) {
-      const int t_l = g0 + lane / boxes, b_l = lane % boxes;
+      const int t_l = g0 + t_mine;
       int row_l = 0;
       if (t_l < n_tiles) {
-        const int j = t_l * KT + b_l * p.box_rows;
+        const int j = (t_first + t_l) * KT + b_l * p.box_rows;
         // a box past the context re-reads the last valid page: its keys are masked anyway,
         // and what it brings is finite
         const int pi = min(j >> p.page_shift, last_page_idx);
@@ -216,27 +268,22 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       }
       const int g_end = min(g0 + group, n_tiles);
       for (int t = g0; t < g_end && ok; ++t) {
-        int rows[8];
-#pragma unroll
-        for (int b = 0; b < 8; ++b) rows[b] = __shfl_sync(0xffffffffu, row_l, ((t - g0) * boxes + b) & 31);
+        const int s = t % STAGES;
         if (lane == 0) {
-          const int s = t % STAGES;
           if (failed || (t >= STAGES && !mbar_wait(&kv_empty[s], ((t / STAGES) - 1) & 1))) {
             failed = 1;
             ok = 0;
           } else {
             mbar_expect_tx(&kv_full[s], 2 * KV_BYTES);
-#pragma unroll
-            for (int b = 0; b < 8; ++b) {
-              if (b < boxes) {
-                tma_load_2d(k_tiles + s * KV_BYTES + b * p.box_rows * HD * 2, &map_k, &kv_full[s], 0, rows[b]);
-                tma_load_2d(v_tiles + s * KV_BYTES + b * p.box_rows * HD * 2, &map_v, &kv_full[s], 0, rows[b]);
-              }
-            }
             issued = t + 1;
           }
         }
         ok = __shfl_sync(0xffffffffu, ok, 0);
+        if (ok && t_l == t) {
+          tma_load_2d(k_tiles + s * KV_BYTES + b_l * p.box_rows * HD * 2, &map_k, &kv_full[s], 0, row_l);
+          tma_load_2d(v_tiles + s * KV_BYTES + b_l * p.box_rows * HD * 2, &map_v, &kv_full[s], 0, row_l);
+        }
+        __syncwarp();
       }
     }
   } else if (warp == SOFTMAX_WARPS + 1) {
@@ -246,7 +293,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       constexpr uint32_t idesc_pv = instr_desc_bf16(QT, HD, 1);   // V tile N-major (rows are keys)
       bool ok = mbar_wait(q_full, 0);
       const uint64_t dq = smem_desc_sw128(smem_u32(q_tile));
-      auto issue_qk = [&](int t) -> bool {  // S[t & 1] = Q K_t^T once tile t has landed
+      auto issue_qk = [&](int t) -> bool {  // S of stream t & 1 = Q K_t^T once tile t has landed
         const int s = t % STAGES;
         if (!mbar_wait(&kv_full[s], (t / STAGES) & 1)) return false;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -258,33 +305,26 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         return true;
       };
       if (ok && n_tiles > 0) ok = issue_qk(0);
-      for (int it = 0; it < n_tiles && ok && !failed; ++it) {
-        const int s = it % STAGES;
-        if (it + 1 < n_tiles) {  // the next tile's scores are computed while this tile's softmax runs
-          ok = issue_qk(it + 1);
-          if (!ok) break;
-        }
+      if (ok && n_tiles > 1) ok = issue_qk(1);
+      for (int t = 0; t < n_tiles && ok && !failed; ++t) {
+        const int s = t % STAGES, st = t & 1;
+        ok = mbar_wait(&p_full[st], (t >> 1) & 1);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint64_t dv = smem_desc_sw128(smem_u32(v_tiles + s * KV_BYTES));
 #pragma unroll
-        for (int st = 0; st < 2; ++st) {
-          ok = mbar_wait(&p_full[2 * st + (it & 1)], (it >> 1) & 1);
-          if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-          for (int kk = 0; kk < 2; ++kk)  // 16 keys = 16 rows of 128 bytes = 8 packed columns of P
-            umma_ts(tmem + COL_O + st * O_COLS, tmem + COL_S + (it & 1) * S_COLS + 32 * st + 8 * kk,
-                    dv + (2048 >> 4) * (2 * st + kk), idesc_pv, (it > 0 || kk > 0) ? 1u : 0u);
-          if (st == 1) umma_commit(&kv_empty[s]);
-          umma_commit(&pv_done[st]);
-        }
-        if (!ok) break;
+        for (int kk = 0; kk < KT / 16; ++kk)  // 16 keys = 16 rows of 128 bytes = 8 packed columns of P
+          umma_ts(tmem + COL_O + st * O_COLS, tmem + COL_S + st * S_COLS + 8 * kk, dv + (2048 >> 4) * kk, idesc_pv,
+                  (t > 1 || kk > 0) ? 1u : 0u);
+        umma_commit(&kv_empty[s]);
+        if (t + 2 < n_tiles) ok = issue_qk(t + 2);
       }
+      if (ok) umma_commit(o_done);
       if (!ok) failed = 2;
     }
     __syncwarp();
   } else {
-    // ---- softmax: threads r and 128 + r own query row r (tensor-memory lane r); the first is
-    // stream 0 (keys 0-31 of every tile), the second stream 1 (keys 32-63)
+    // ---- softmax: threads r and 128 + r own query row r (tensor-memory lane r), the first for even tiles
     const int st = warp >> 2, wq = warp & 3;
     const int r = wq * 32 + lane;
     const int qpos = pos0 + q0 + r;
@@ -295,93 +335,127 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     const lse::SoftCap softcap(CAP ? a.softcap : 0.f);
     float m_run = -INFINITY, l_run = 0.f;
     bool ok = true;
-    for (int it = 0; it < n_tiles && !failed; ++it) {
-      ok = mbar_wait(&s_full[it & 1], (it >> 1) & 1);
+    const uint32_t s_col = lane_base + COL_S + st * S_COLS;
+    for (int t = st, round = 0; t < n_tiles; t += 2, ++round) {
+      ok = mbar_wait(&s_full[st], round & 1);
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t s_buf = lane_base + COL_S + (it & 1) * S_COLS + 32 * st;
-      uint32_t sv[32];
-      tmem_ld32(s_buf, sv);
+      uint32_t sa[32], sb[32];  // the keys of the tile's first and second half
+      tmem_ld32(s_col, sa);
+      tmem_ld32(s_col + 32, sb);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       if constexpr (CAP) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) sv[j] = __float_as_uint(softcap(__uint_as_float(sv[j]) * a.scale));
+        for (int j = 0; j < 32; ++j) {
+          sa[j] = __float_as_uint(softcap(__uint_as_float(sa[j]) * a.scale));
+          sb[j] = __float_as_uint(softcap(__uint_as_float(sb[j]) * a.scale));
+        }
       }
-      const int k0 = it * KT + 32 * st;
-      // four independent chains for the maximum and for the sum: a single chain of dependent
-      // operations would leave the warp waiting on its own results
-      float mx4[4] = {m_run, -INFINITY, -INFINITY, -INFINITY};
-      if (k0 + 31 > pos0 + q0) {  // keys that reach the diagonal: mask per element
+      const int k0 = (t_first + t) * KT;
+      if (k0 + KT - 1 > pos0 + q0) {  // keys that reach the diagonal: mask per element
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
-          const float v = (k0 + j <= qpos) ? __uint_as_float(sv[j]) : -INFINITY;
-          sv[j] = __float_as_uint(v);
-          mx4[j & 3] = fmaxf(mx4[j & 3], v);
+          sa[j] = (k0 + j <= qpos) ? sa[j] : 0xff800000u;  // -inf
+          sb[j] = (k0 + 32 + j <= qpos) ? sb[j] : 0xff800000u;
         }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) mx4[j & 3] = fmaxf(mx4[j & 3], __uint_as_float(sv[j]));
       }
+      // independent chains for the maximum and for the sum: a single chain of dependent
+      // operations would leave the warp waiting on its own results
+      float mx4[4] = {m_run, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+      for (int j = 0; j < 32; ++j)
+        mx4[j & 3] = fmaxf(fmaxf(mx4[j & 3], __uint_as_float(sa[j])), __uint_as_float(sb[j]));
       const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
       // The reference maximum of the exponent moves only when some row of the warp has outgrown
       // it by a factor 2^8: until then P may reach 256 (exact enough in bfloat16, sums are
-      // float32) and O needs no rescaling, so most tiles neither touch O nor wait for the P V
-      // before them. (-inf) - (-inf) is NaN and compares false: a row without keys asks for nothing.
+      // float32) and O needs no rescaling, so most tiles do not touch O.
+      // (-inf) - (-inf) is NaN and compares false: a row without keys asks for nothing.
       const bool grow = __any_sync(0xffffffffu, (mx - m_run) * sl2 > 8.f);
       const float m_new = grow ? mx : m_run;
       const float m_fin = (m_new == -INFINITY) ? 0.f : m_new;
-      const float corr = grow ? ex2((m_run - m_fin) * sl2) : 1.f;  // m_run = -inf gives 0
       const float ms = m_fin * sl2;
-      m_run = m_new;
-      float sum4[4] = {0.f, 0.f, 0.f, 0.f};
-      uint32_t pk[16];
+      if (grow) {
+        const float corr = ex2((m_run - m_fin) * sl2);  // m_run = -inf gives 0
+        m_run = m_new;
+        l_run *= corr;
+        if (round > 0) {  // (this stream's P V of before is complete: its S came after it)
+          uint32_t ov[16];
+#pragma unroll 1
+          for (int h = 0; h < 4; ++h) {
+            tmem_ld16(o_col + 16 * h, ov);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const float p0 = ex2(fmaf(__uint_as_float(sv[2 * j]), sl2, -ms));
-        const float p1 = ex2(fmaf(__uint_as_float(sv[2 * j + 1]), sl2, -ms));
-        sum4[j & 3] += p0 + p1;
-        pk[j] = pack2(p0, p1);  // element 2j in the low half, 2j+1 in the high half
-      }
-      const float sum = (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
-      l_run = l_run * corr + sum;
-      if (it > 0 && grow) {
-        // this stream's O of the tiles so far must be complete before it is rescaled
-        ok = mbar_wait(&pv_done[st], (it - 1) & 1);
-        if (!ok) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        uint32_t ov[16];
-#pragma unroll
-        for (int h = 0; h < 4; ++h) {
-          tmem_ld16(o_col + 16 * h, ov);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-          for (int j = 0; j < 16; ++j) ov[j] = __float_as_uint(__uint_as_float(ov[j]) * corr);
-          tmem_st16(o_col + 16 * h, ov);
+            for (int j = 0; j < 16; ++j) ov[j] = __float_as_uint(__uint_as_float(ov[j]) * corr);
+            tmem_st16(o_col + 16 * h, ov);
+          }
         }
       }
-      tmem_st16(s_buf, pk);
+      float2 sum2[2] = {make_float2(l_run, 0.f), make_float2(0.f, 0.f)};
+      const float2 sl2x2 = make_float2(sl2, sl2), msx2 = make_float2(-ms, -ms);
+      auto exponentials = [&](const uint32_t (&sv)[32], uint32_t col) {
+        uint32_t pk[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const float2 x = fma2(make_float2(__uint_as_float(sv[2 * j]), __uint_as_float(sv[2 * j + 1])), sl2x2, msx2);
+          const float2 e = make_float2(ex2(x.x), ex2(x.y));
+          sum2[j & 1] = add2(sum2[j & 1], e);
+          pk[j] = pack2(e.x, e.y);  // element 2j in the low half, 2j+1 in the high half
+        }
+        tmem_st16(col, pk);
+      };
+      exponentials(sa, s_col);
+      exponentials(sb, s_col + 16);
+      const float2 sum = add2(sum2[0], sum2[1]);
+      l_run = sum.x + sum.y;
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      // Even and odd tiles arrive on different barriers. A warp that does not wait for the P V
-      // of the tile before may be a tile ahead of the other warps of its stream, and of the MMA
-      // thread; it can be two tiles ahead of neither, because S of tile it + 2 is computed only
-      // after the MMA thread has seen every arrival of tile it. So an arrival is never counted
-      // for a phase that is still collecting an earlier tile, and the MMA thread never finds a
-      // barrier two phases on.
       __syncwarp();
-      if (lane == 0) mbar_arrive(&p_full[2 * st + (it & 1)]);
+      if (lane == 0) mbar_arrive(&p_full[st]);
     }
     if (!ok) failed = 3;
     // ---- epilogue: the two streams of a row are merged; each of its threads writes 32 head dims
     pair_m[st][r] = m_run;
     pair_l[st][r] = l_run;
     if (ok && !failed && n_tiles > 0) {
-      ok = mbar_wait(&pv_done[0], (n_tiles - 1) & 1) && mbar_wait(&pv_done[1], (n_tiles - 1) & 1);
+      ok = mbar_wait(o_done, 0);
       if (!ok) failed = 4;
     }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("bar.sync 1, %0;" ::"n"(SOFTMAX_WARPS * 32) : "memory");  // the softmax warps only
-    if (ok && !failed) {
+    if (PARTS > 1) {
+      // every block of the cluster gets the head dims that it merges, and every row's maximum and sum
+      constexpr int DP = HD / PARTS, ROW = inbox_row(PARTS);
+      const float m0 = pair_m[0][r], m1 = pair_m[1][r];
+      const bool usable = ok && !failed && n_tiles > 0;
+      const float mm = usable ? fmaxf(m0, m1) : -INFINITY;
+      const float w0 = (!usable || m0 == -INFINITY) ? 0.f : ex2((m0 - mm) * sl2);
+      const float w1 = (!usable || m1 == -INFINITY) ? 0.f : ex2((m1 - mm) * sl2);
+      const float l = usable ? pair_l[0][r] * w0 + pair_l[1][r] * w1 : 0.f;
+      const uint32_t here = smem_u32(inbox);
+      cluster_arrive();
+      cluster_wait();  // no block of the cluster reads its tiles any more
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        uint32_t oa[16], ob[16];
+        tmem_ld16(lane_base + COL_O + 32 * st + 16 * h, oa);
+        tmem_ld16(lane_base + COL_O + O_COLS + 32 * st + 16 * h, ob);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int j = 0; j < 16; j += 4) {
+          float o[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            o[e] = (w0 != 0.f ? __uint_as_float(oa[j + e]) * w0 : 0.f) + (w1 != 0.f ? __uint_as_float(ob[j + e]) * w1 : 0.f);
+          const int d = 32 * st + 16 * h + j;
+          store_peer4(peer_address(here + (uint32_t)(((part * QT + r) * ROW + d % DP) * 4), d / DP), o[0], o[1], o[2], o[3]);
+        }
+      }
+      if (st == 0) {
+#pragma unroll
+        for (int z = 0; z < PARTS; ++z)
+          store_peer2(peer_address(here + (uint32_t)((PARTS * QT * ROW + (part * QT + r) * 2) * 4), z), mm, l);
+      }
+    } else if (ok && !failed) {
       const float m0 = pair_m[0][r], m1 = pair_m[1][r];
       const float mm = fmaxf(m0, m1);
       const float w0 = (m0 == -INFINITY) ? 0.f : ex2((m0 - mm) * sl2);
@@ -402,7 +476,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
             float o[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e)
-              o[e] = __uint_as_float(oa[j + e]) * f0 + __uint_as_float(ob[j + e]) * f1;
+              o[e] = (f0 != 0.f ? __uint_as_float(oa[j + e]) * f0 : 0.f) +
+                     (f1 != 0.f ? __uint_as_float(ob[j + e]) * f1 : 0.f);  // (O of a stream without tiles was never written)
             uint4 w;
             w.x = pack2(o[0], o[1]);
             w.y = pack2(o[2], o[3]);
@@ -412,6 +487,42 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
           }
         }
       }
+    }
+  }
+  if constexpr (PARTS > 1) {
+    __syncwarp();
+    if (warp >= SOFTMAX_WARPS) {  // (the softmax warps did before they wrote)
+      cluster_arrive();
+      cluster_wait();
+    }
+    cluster_arrive();
+    cluster_wait();
+    constexpr int DP = HD / PARTS, ROW = inbox_row(PARTS), PIECES = DP / 8;
+    const float sl2 = (CAP ? 1.f : a.scale) * 1.4426950408889634f;
+    const float2* ml = reinterpret_cast<const float2*>(inbox + PARTS * QT * ROW);
+    for (int i = threadIdx.x; i < rows_here * PIECES; i += THREADS) {
+      const int r = i / PIECES, d = (i - r * PIECES) * 8;
+      float top = -INFINITY;
+#pragma unroll
+      for (int z = 0; z < PARTS; ++z) top = fmaxf(top, ml[z * QT + r].x);
+      float l = 0.f, o[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int z = 0; z < PARTS; ++z) {
+        const float2 v = ml[z * QT + r];
+        const float w = v.x == -INFINITY ? 0.f : ex2((v.x - top) * sl2);
+        l = fmaf(v.y, w, l);
+        const float4* src = reinterpret_cast<const float4*>(inbox + (z * QT + r) * ROW + d);
+        const float4 x = src[0], y = src[1];
+        o[0] = fmaf(x.x, w, o[0]); o[1] = fmaf(x.y, w, o[1]); o[2] = fmaf(x.z, w, o[2]); o[3] = fmaf(x.w, w, o[3]);
+        o[4] = fmaf(y.x, w, o[4]); o[5] = fmaf(y.y, w, o[5]); o[6] = fmaf(y.z, w, o[6]); o[7] = fmaf(y.w, w, o[7]);
+      }
+      const float inv = l > 0.f ? 1.f / l : 0.f;
+      uint4 w;
+      w.x = pack2(o[0] * inv, o[1] * inv);
+      w.y = pack2(o[2] * inv, o[3] * inv);
+      w.z = pack2(o[4] * inv, o[5] * inv);
+      w.w = pack2(o[6] * inv, o[7] * inv);
+      *reinterpret_cast<uint4*>((bf16*)a.out + (size_t)(q_start + q0 + r) * a.out_row_stride + (size_t)head * HD + part * DP + d) = w;
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -436,6 +547,19 @@ inline bool supported(const LseAttnArgs* a) {
          (a->q_row_stride % 8) == 0 && (a->out_row_stride % 8) == 0;
 }
 
+template <bool CAP, int PARTS>
+inline int launch_prefill_parts(const LseAttnArgs* a, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
+                                const Params& p, cudaStream_t stream) {
+  constexpr int smem = Q_BYTES + 2 * STAGES * KV_BYTES + (2 * STAGES + 6) * 8 + 16 + 1024;
+  static const cudaError_t configured =
+      cudaFuncSetAttribute(prefill_tc_kernel<CAP, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (configured != cudaSuccess) return LSE_LAUNCH_FAILED;
+  const dim3 grid(a->num_heads * PARTS, a->num_tiles);
+  return lse::launch_clusters(prefill_tc_kernel<CAP, PARTS>, grid, THREADS, PARTS, smem, stream, mq, mk, mv, p) == cudaSuccess
+             ? LSE_OK
+             : LSE_LAUNCH_FAILED;
+}
+
 // total_rows: rows of the query tensor; pool_rows: pages * kv_heads * page_tokens.
 template <bool CAP>
 inline int launch_prefill_form(const LseAttnArgs* a, long long total_rows, long long pool_rows,
@@ -452,18 +576,19 @@ inline int launch_prefill_form(const LseAttnArgs* a, long long total_rows, long 
   p.page_shift = 0;
   while ((1 << p.page_shift) < a->page_tokens) ++p.page_shift;
   p.error_flag = error_flag;
-  constexpr int smem = Q_BYTES + 2 * STAGES * KV_BYTES + (2 * STAGES + 9) * 8 + 16 + 1024;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(prefill_tc_kernel<CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-        cudaSuccess)
-      return LSE_LAUNCH_FAILED;
-    configured = true;
+  // Two blocks run on an SM at a time. A grid that leaves half of these places empty is as slow as its longest block,
+  // so the keys of a (query tile, head) are shared by a cluster. Measured alone, 1 / 2 / 4 blocks each, us:
+  // 9 blocks, 512 keys 16.4 / 14.6 / 14.5, 4000 keys 51 / 33 / 25; 32 blocks, 2048 keys 31 / 23 / 21; 72 blocks, 1024
+  // keys 21 / 18 / 25; 128 blocks, 512 keys 16.4 / 17.4 / 29, 2000 keys 32 / 27 / 39; 144 blocks, 8184 keys 94 / 60 / 88;
+  // 256 blocks, 1000 keys 23 / 29 / 51 (a further wave). The longest context is known here as what a table holds.
+  const long long blocks = (long long)a->num_heads * a->num_tiles;
+  const long long keys = (long long)a->table_stride * a->page_tokens;
+  const int want = keys <= 512 || blocks > 148 ? 1 : blocks <= 32 ? 4 : 2;
+  switch (want) {
+    case 1: return launch_prefill_parts<CAP, 1>(a, mq, mk, mv, p, stream);
+    case 2: return launch_prefill_parts<CAP, 2>(a, mq, mk, mv, p, stream);
+    default: return launch_prefill_parts<CAP, 4>(a, mq, mk, mv, p, stream);
   }
-  dim3 grid(a->num_heads, a->num_tiles);
-  return lse::launch(prefill_tc_kernel<CAP>, grid, THREADS, smem, stream, mq, mk, mv, p) == cudaSuccess
-             ? LSE_OK
-             : LSE_LAUNCH_FAILED;
 }
 
 inline int launch_prefill(const LseAttnArgs* a, long long total_rows, long long pool_rows,

@@ -376,6 +376,20 @@ def test_rope_kv_write_and_attention_mixed_batch(ops, dtype, nq, nk, D, page):
     close(got, ref, dtype, atol32=1e-5, rel16=0.02)
 
 
+@pytest.mark.parametrize("page", [8, 16, 64])
+@pytest.mark.parametrize("nq,nk,q_lens,ctx_lens", [
+    (2, 1, [3, 130, 2, 64], [515, 900, 2, 65]),   # few blocks: four share a tile's keys, of some tiles only one has any
+    (24, 8, [129, 2, 128], [640, 2, 449]),        # two share them
+    (3, 3, [127, 129], [512, 129]),               # short tables: nothing is shared
+    (40, 8, [200, 300], [700, 300])])             # many blocks: nothing is shared
+def test_prefill_attention_shared_by_clusters(ops, nq, nk, q_lens, ctx_lens, page):
+    """float32 sums of bfloat16 probabilities and values: as the tolerance of the other bfloat16 attention tests."""
+    case = paged_case(len(q_lens), q_lens, ctx_lens, nq, nk, 64, page, torch.bfloat16, seed=nq)
+    got, ref, _ = run_attention(ops, case, nq, nk, 64, page, 0, 1024)
+    close(got, ref, "bfloat16", rel16=0.02)
+    ops.check_kernel_errors()
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("window", [1, 5, 64, 100])
 def test_attention_window_edges(ops, dtype, window):
