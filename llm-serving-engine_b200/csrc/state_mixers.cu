@@ -7,6 +7,7 @@
 // whose first row of this step is at position 0 starts from zeros, whatever its slot holds.
 #include "common.cuh"
 #include "kernels.h"
+#include "linear_chunks.cuh"
 
 namespace lse {
 
@@ -470,7 +471,9 @@ __global__ void norm_rope_kv_write_kernel(const float* __restrict__ qkv, T* __re
 // shared memory per pass. The state is stored transposed, [slot][head][value_dim][key_dim]: a
 // thread's rows are contiguous there.
 //
-// A portion longer than L tokens is cut into chunks of L that run side by side, in three launches:
+// A portion longer than L tokens is cut into chunks of L. With a decay per head and key and value sizes that are
+// multiples of 4 up to 128 they run as matrix products (linear_chunks.cuh, 149 against 269 us at 16 heads of 128 x 128
+// and 2048 tokens); otherwise side by side here, in three launches:
 //   A  every chunk steps through its tokens from a zero state (the first chunk from the request's
 //      state) and leaves its outputs and its final state (chunk c: E_c) in a scratch;
 //   B  the chunks' states are chained, element by element: F_0 = E_0, F_c = decay^len_c F_{c-1} + E_c;
@@ -497,6 +500,7 @@ struct LinAttnArgs {
   float key_scale;
   int P, CB;              // lanes per column; columns per block
   int L;                  // chunk length
+  int short_only;         // 1: sequences of more than one chunk are served elsewhere
   int phase;              // 0: launch A, 2: launch C
   // a decay per key channel and token instead of decay[h]: alpha = sigmoid(z)^inv_root
   const float* gate_z;    // [T, gate_stride], heads x dk logits per row; null: the fixed decays
@@ -552,7 +556,7 @@ __global__ void __launch_bounds__(LA_THREADS, MODE == 0 ? 0 : 3) decay_linear_at
   const int num_chunks = (n + L - 1) / L;
   const bool add_pass = MODE == 0 ? a.phase == 2 : MODE == 2;
   const int c = blockIdx.y + (add_pass ? 1 : 0);
-  if (c >= num_chunks) {
+  if (c >= num_chunks || (a.short_only && num_chunks > 1)) {
     pdl_wait();  // no block leaves before the kernels before this one are done: the next kernel counts on it
     return;
   }
@@ -1073,6 +1077,21 @@ extern "C" int lse_decay_linear_attention(const float* proj, long long stride, f
 #undef LSE_LA_KERNEL
   a.L = lse_linear_attention_chunk();
   a.phase = 0;
+  a.short_only = 0;
+  if (!gated && max_chunks > 1) {
+    // a decay per head: the chunks of long portions as matrix products (linear_chunks.cuh), where the sizes allow it
+    lac::Args m;
+    m.proj = proj; m.stride = stride; m.out = out; m.state = state; m.chunks = chunks; m.decay = decay;
+    m.cu_q = cu_q; m.ctx_lens = ctx_lens; m.slots = slots; m.cos = cos; m.sin = sin; m.H = H; m.dk = dk; m.dv = dv;
+    m.rot = rot; m.silu = silu; m.key_scale = key_scale; m.query_scale = query_scale;
+    static_assert(lac::L == 64, "the chunk of lse_linear_attention_chunk()");
+    if (lac::serves(m)) {
+      const int code = lac::run(m, num_seqs, max_chunks, stream);
+      if (code != LSE_OK || (num_seqs == 1 && total_rows > lac::L)) return code;  // (the one sequence is a long one)
+      a.short_only = 1;
+      max_chunks = 1;
+    }
+  }
   const int slices = (dv + a.CB - 1) / a.CB;
   const int tile = gated ? LA_TT_GATED : LA_TT;
   const size_t smem =

@@ -144,6 +144,34 @@ def test_linear_attention_chunked_and_short_sequences_in_one_step(ops):
     close(out[300:301], ref1[7:], 2e-5, "1")
 
 
+@pytest.mark.parametrize("H,dk,dv,rot,silu", [(2, 4, 4, 0, False), (1, 64, 68, 12, True), (2, 68, 64, 68, False),
+                                              (3, 128, 128, 64, True), (1, 124, 132, 0, False), (1, 132, 124, 0, True)])
+def test_linear_attention_chunk_products_at_their_edges(ops, H, dk, dv, rot, silu):
+    """Sizes at and beyond the edges of the kernel's tiles (64, 128); a chunk of one token and whole chunks, beside
+    sequences of at most a chunk, with and without a state before them."""
+    decay = [0.999, 0.9, 0.2][:H]
+    width = 2 * H * dk + H * dv
+    width += -width % 4
+    lens, pos = [65, 64, 128, 1, 193], [0, 0, 30, 5, 7]
+    cos, sin = rotary_tables(rot, 1e4, 256) if rot else (None, None)
+    kw = dict(num_heads=H, key_dim=dk, value_dim=dv, decay=torch.tensor(decay).cuda(),
+              activation="silu" if silu else "none", key_scale=dk ** -0.5, cos=cos, sin=sin)
+    seqs = [rnd(p + n, width, seed=40 + i, scale=0.7) for i, (n, p) in enumerate(zip(lens, pos))]
+    state = torch.full((7, H, dv, dk), 1e4).cuda()
+    slots = [3, 0, 5, 1, 2]
+    for s, p, slot in zip(seqs, pos, slots):
+        for t in range(p):  # token by token: the recurrence
+            ops.decay_linear_attention(s[t : t + 1].cuda(), state=state, step=batch([1], [t], [slot]), **kw)
+    rows = torch.cat([s[p:] for s, p in zip(seqs, pos)])
+    out = ops.decay_linear_attention(rows.cuda(), state=state, step=batch(lens, pos, slots), **kw)
+    at = 0
+    for s, p, n in zip(seqs, pos, lens):
+        ref = linear_attention_reference(s, H, dk, dv, decay, silu, rot, 1e4, dk ** -0.5)[p:]
+        close(out[at : at + n], ref, 2e-5, str(n))
+        at += n
+    assert bool((state[[4, 6]] == 1e4).all())
+
+
 def test_linear_attention_keeps_a_key_from_far_away(ops):
     """One early key/value pair is made large; with a decay close to one it must still be most of
     the output 700 tokens later (and gone with a small decay)."""
