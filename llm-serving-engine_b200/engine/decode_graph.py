@@ -449,7 +449,7 @@ class DecodeGraphs:
         plans = self._plans_mixed(shape, padded)
         # context partitions as for the next power of two of the longest context: fewer shapes
         max_ctx = pow2_at_least(int(arrays["ctx_lens"][:B].max())) if B else 1
-        splits = runner.ops.decode_splits(B, self.min_kv_heads, max_ctx) if B else 1
+        splits = runner.ops.decode_splits(B, self.min_kv_heads, max_ctx, runner.dtype) if B else 1
         # unsampled and padding rows are greedy, so the one-block kernel is always there
         kinds = (sample_kinds(r.params for r in rows) | 1) if simple else 0
         key = (B, P, TP, splits, simple, kinds)
@@ -586,7 +586,7 @@ class DecodeGraphs:
             raise ValueError("these rows need a sampler and cannot run ahead")
         ahead = 0 if ahead_of is None else 1
         max_ctx = 1 + ahead + max(runner.manager.held[e.rid].computed for e in entries)
-        splits = runner.ops.decode_splits(B, self.min_kv_heads, max_ctx)
+        splits = runner.ops.decode_splits(B, self.min_kv_heads, max_ctx, runner.dtype)
         # padding rows are greedy, so a padded batch always holds the one-block kernel
         kinds = (sample_kinds(r.params for r in rows) | (1 if B > n else 0)) if simple else 0
         key = (B, splits, simple, kinds)
@@ -608,7 +608,7 @@ class DecodeGraphs:
         n = len(entries)
         B = self.padded(n)
         max_ctx = 1 + max(runner.manager.held[e.rid].computed for e in entries)
-        splits = runner.ops.decode_splits(B, self.min_kv_heads, max_ctx)
+        splits = runner.ops.decode_splits(B, self.min_kv_heads, max_ctx, runner.dtype)
         key = (B, splits, False, 0)
         g = self.graphs.get(key)
         if g is None:

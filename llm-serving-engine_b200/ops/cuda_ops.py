@@ -91,7 +91,7 @@ _BLOCK_START_KEYS = 130
 _MERGE_KEYS_PER_SPLIT = 4
 
 
-def choose_decode_splits(pairs: int, max_ctx: int, num_sms: int, blocks_per_sm: int) -> int:
+def choose_decode_splits(pairs: int, max_ctx: int, num_sms: int, blocks_per_sm: int, min_keys: int = 128) -> int:
     """Context partitions per (sequence, key/value head) for ``pairs`` such pairs.
 
     The kernel runs one block per (partition, pair); ``blocks_per_sm * num_sms`` of them run at a
@@ -99,15 +99,15 @@ def choose_decode_splits(pairs: int, max_ctx: int, num_sms: int, blocks_per_sm: 
     not by how many blocks share the SM, and a wave that is part empty takes as long as a full
     one: 12 sequences x 32 heads cut in 3 make 1152 blocks for 1036 places and took 49 us where
     24 sequences took 79. So the number of partitions is the one that minimises
-    ``waves * (keys per block + a block's fixed cost)``, among partitions of 128 keys or more
-    (measured at one sequence of 2176 keys: 8 partitions 13.3 us, 16 10.9, 28 11.9, 34 12.1).
+    ``waves * (keys per block + a block's fixed cost)``, among partitions of ``min_keys`` keys or more
+    (128: measured at one sequence of 2176 keys: 8 partitions 13.3 us, 16 10.9, 28 11.9, 34 12.1).
     The context is rounded up to a power of two first, so that the choice (which captured graphs
     are keyed on) does not flicker from step to step. Without a known occupancy: about six blocks
     per SM.
     """
     if pairs <= 0:
         return 1
-    most = int(max(1, min((max_ctx + 127) // 128, 64)))
+    most = int(max(1, min((max_ctx + min_keys - 1) // min_keys, 64)))
     if blocks_per_sm <= 0:
         want = max(1, (6 * num_sms + pairs - 1) // pairs)
         return int(min(want, most))
@@ -446,9 +446,12 @@ class CudaOps:
             "decode_seqs": np.asarray(decode, dtype=np.int32),
         }
 
-    def decode_splits(self, num_decode, num_kv_heads, max_ctx):
-        """Context partitions per (sequence, head) for a step of single tokens."""
-        return choose_decode_splits(num_decode * num_kv_heads, max_ctx, self.num_sms, self.decode_blocks_per_sm)
+    def decode_splits(self, num_decode, num_kv_heads, max_ctx, dtype=None):
+        """Context partitions per (sequence, head) for a step of single tokens. The float32 kernel has 16 keys of a
+        block in flight where the bfloat16 one has 64, so its partitions may be shorter: 6 sequences of 300 keys, 9
+        heads on 3 key heads, 24 steps of 30 layers in partitions of 128 / 64 / 32 / 16 keys 55.2 / 52.5 / 51.5 / 51.3 ms."""
+        return choose_decode_splits(num_decode * num_kv_heads, max_ctx, self.num_sms, self.decode_blocks_per_sm,
+                                    32 if dtype == torch.float32 else 128)
 
     def paged_attention(self, q, *, num_heads, num_kv_heads, head_dim, scale, window, k_pages,
                         v_pages, block_tables, page_tokens, step, plan, head_scale=None, slopes=None,
@@ -463,7 +466,7 @@ class CudaOps:
         n_tiles = int(plan["tiles"].shape[0])
         n_dec = int(plan["decode_seqs"].shape[0])
         splits = step.decode_splits if step.decode_splits else self.decode_splits(
-            n_dec, num_kv_heads, step.max_decode_ctx)
+            n_dec, num_kv_heads, step.max_decode_ctx, q.dtype)
         scratch = None
         if n_dec and splits > 1:
             self.reserve_attention_scratch(head_dim, n_dec, num_heads, splits)
