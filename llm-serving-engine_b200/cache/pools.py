@@ -106,11 +106,13 @@ class CachePools:
                 self._states_of.setdefault(cid, []).append((gi, li))
         self._order: dict[int, list[tuple[tuple, object]]] = {}
         self._state_views: dict[int, tuple] = {}
+        self._views: dict[tuple, CacheView] = {}  # the tensors are made once, and so are the views of them
 
     def declare_order(self, needs: dict[int, object]) -> None:
         """Remember in which order each cache layer declared its states, so that ``view().states``
         follows it (states of equal shape keep their order within their group anyway)."""
         self._state_views.clear()
+        self._views.clear()
         for cid, need in needs.items():
             self._order[cid] = [(tuple(n.shape), n.dtype) for n in flatten_needs(need)
                                 if isinstance(n, StateNeed)]
@@ -132,6 +134,12 @@ class CachePools:
         return got
 
     def view(self, cache_id: int, writes: bool) -> CacheView:
+        got = self._views.get((cache_id, writes))
+        if got is None:
+            got = self._views[cache_id, writes] = self._make_view(cache_id, writes)
+        return got
+
+    def _make_view(self, cache_id: int, writes: bool) -> CacheView:
         where = self._pages_of.get(cache_id)
         states = self._states(cache_id)
         first = states[0] if states else None

@@ -3,9 +3,12 @@
 // PyTorch's current CUDA stream. Attention kernels live in one shared library per head size,
 // loaded here with dlopen.
 #include <ATen/cuda/CUDAContext.h>
+#include <cublas_v2.h>
 #include <dlfcn.h>
 #include <torch/extension.h>
 
+#include <algorithm>
+#include <climits>
 #include <map>
 #include <optional>
 #include <string>
@@ -232,6 +235,30 @@ void poly_norm(const Tensor& z, const Tensor& coef, double eps, Tensor& out) {
   done(lse_poly_norm(z.data_ptr(), dtype_code(z, "z"), coef.data_ptr<float>(), (float)eps, out.data_ptr(),
                      dtype_code(out, "out"), (int)z.size(0), (int)z.size(1), stream()),
        "poly_norm");
+}
+
+// out = alpha a w^T (+ out) by the library, float32 sums, as torch.mm and torch.addmm call it by default: the same
+// function with the same arguments, without the views, the argument parsing and the dispatch in front of it.
+void gemm_bf16_library(const Tensor& a, const Tensor& w, Tensor& out, double alpha, bool accumulate) {
+  for (const Tensor* t : {&a, &w}) {
+    TORCH_CHECK(t->is_cuda() && t->is_contiguous() && t->dim() == 2 && t->scalar_type() == torch::kBFloat16,
+                "gemm_bf16_library: a and w must be contiguous bfloat16 CUDA matrices");
+  }
+  TORCH_CHECK(out.is_cuda() && out.is_contiguous() && out.dim() == 2, "gemm_bf16_library: out must be a contiguous CUDA matrix");
+  const int64_t T = a.size(0), N = w.size(0), K = a.size(1);
+  TORCH_CHECK(T > 0 && N > 0 && K > 0 && w.size(1) == K && out.size(0) == T && out.size(1) == N,
+              "gemm_bf16_library: need a [T, K], w [N, K], out [T, N]");
+  TORCH_CHECK(out.scalar_type() == torch::kBFloat16 || out.scalar_type() == torch::kFloat32,
+              "gemm_bf16_library: out must be bfloat16 or float32");
+  TORCH_CHECK(std::max({T, N, K}) <= INT_MAX, "gemm_bf16_library: sizes beyond 32 bits");
+  const float one = (float)alpha, beta = accumulate ? 1.f : 0.f;
+  cublasHandle_t handle = at::cuda::getCurrentCUDABlasHandle();  // on the current stream, with torch's workspace
+  const cublasStatus_t status =
+      cublasGemmEx(handle, CUBLAS_OP_T, CUBLAS_OP_N, (int)N, (int)T, (int)K, &one, w.const_data_ptr(), CUDA_R_16BF, (int)K,
+                   a.const_data_ptr(), CUDA_R_16BF, (int)K, &beta, out.data_ptr(),
+                   out.scalar_type() == torch::kFloat32 ? CUDA_R_32F : CUDA_R_16BF, (int)N, CUBLAS_COMPUTE_32F,
+                   CUBLAS_GEMM_DEFAULT_TENSOR_OP);
+  TORCH_CHECK(status == CUBLAS_STATUS_SUCCESS, "gemm_bf16_library: the library failed with status ", num((int)status));
 }
 
 void gemm_f32(const Tensor& a, const Tensor& w, const OptTensor& bias, Tensor& out) {
@@ -1420,6 +1447,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("limit") = 0.0, py::arg("col0") = 0);
   m.def("poly_norm", &poly_norm);
   m.def("gemm_f32", &gemm_f32);
+  m.def("gemm_bf16_library", &gemm_bf16_library);
   m.def("gemm_bf16_skinny", &gemm_bf16_skinny);
   m.def("gemm_bf16_skinny_max_rows", &gemm_bf16_skinny_max_rows);
   m.def("fixed_to_float", &fixed_to_float);

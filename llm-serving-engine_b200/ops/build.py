@@ -144,7 +144,7 @@ def load_core(verbose: bool = False):
                         extra_include_paths=[str(CSRC)],
                         extra_cflags=["-O2", "-std=c++17"],
                         extra_cuda_cflags=ARCH_FLAGS + NVCC_FLAGS,
-                        extra_ldflags=["-ldl"],
+                        extra_ldflags=["-ldl", "-lcublas"],
                         build_directory=str(folder),
                         with_cuda=True,
                         verbose=verbose,
