@@ -1834,7 +1834,7 @@ extern "C" int lse_attn_prefill(const LseAttnArgs* a, cudaStream_t stream) {
     else prefill_simt_kernel<float, false><<<grid, 128, 0, stream>>>(*a, ps);
 #if LSE_HEAD_DIM == 64
   } else if (a->force_simt == 0 && a->num_rows > 0 && a->num_pages > 0 && atc::supported(a) &&
-             !(a->head_scale || a->slopes || a->chunk > 0 || a->sinks || a->keep_first > 0 || a->out_f32)) {
+             !(a->head_scale || a->slopes || (a->keep_first > 0 && a->window > 0) || a->out_f32)) {
     // 128-row tiles, like the mma.sync kernel
     return atc::launch_prefill(a, a->num_rows, a->num_pages * a->num_kv_heads * a->page_tokens,
                                a->error_flag, stream);

@@ -53,7 +53,8 @@ struct LseAttnArgs {
   const float* rope_cos;
   const float* rope_sin;
   // Options of the score, all off when null / 0. With any of them on, the CUDA-core kernels and
-  // the mma.sync kernel for portions serve the call (lse_attn_decode_takes_sums() does not hold).
+  // the mma.sync kernel for portions serve the call (lse_attn_decode_takes_sums() does not hold); chunks and
+  // sinks, like a window, are also served by the tcgen05 kernel for portions (head size 64).
   //   s_ij = softcap(scale * head_scale[h] * q_i . k_j) - slopes[h] * (i - j)
   //   chunk > 0: query i reads key j only if i / chunk == j / chunk (absolute positions)
   const float* head_scale;  // [num_heads] or null

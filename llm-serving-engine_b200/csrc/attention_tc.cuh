@@ -1,5 +1,6 @@
 // Flash-style causal attention for portions of prompts on the 5th-generation tensor cores
-// (head size 64, bfloat16, no window, page size a power of two >= 8).
+// (head size 64, bfloat16, page size a power of two >= 8; everything before a row, a window or the row's chunk; soft
+// caps and sinks).
 //
 // One block = 128 query rows of one head. Per tile of 64 keys:
 //   S = Q K^T        tcgen05.mma, A = Q tile and B = K tile in shared memory (both K-major, TMA with
@@ -25,6 +26,7 @@
 // tile; issued by one lane they were what a tile waited for. 2040 rows behind 6144 keys, 9 heads: 123 us (one lane
 // issuing, both streams on halves of one tile) -> 94 us -> 60 us with the keys shared by two blocks (exp unit alone:
 // 29 us); 2048 rows behind 4096 keys, 32 heads: 166 -> 141 us (75 us); 2048 rows alone, 32 heads: 45 -> 47 us (15 us).
+// 2048 rows, 32 heads, a window of 1024 with sinks: 41 us, chunks of 512: 29 us (mma.sync kernel: 125, 59).
 #pragma once
 
 #include "attention_args.h"
@@ -166,8 +168,16 @@ __host__ __device__ constexpr int inbox_bytes(int parts) {
   return parts > 1 ? parts * QT * (inbox_row(parts) + 2) * 4 : 0;
 }
 
+// First key that a query at position qpos may read (window and chunk together); it never moves back.
+__device__ __forceinline__ int first_local_key(const LseAttnArgs& a, int qpos) {
+  const int lo = a.window > 0 ? max(0, qpos - a.window + 1) : 0;
+  return a.chunk > 0 ? max(lo, qpos / a.chunk * a.chunk) : lo;
+}
+
 // CAP: the scores are scaled and soft-capped as they leave tensor memory. PARTS: blocks per (query tile, head).
-template <bool CAP, int PARTS>
+// LOCAL: a window or chunks. Keys before a row's first are masked like those behind it; the first tile starts on a
+// multiple of 64, and what a page that is no longer held would bring is read from the first page that is.
+template <bool CAP, int PARTS, bool LOCAL>
 __global__ void __launch_bounds__(THREADS, 2)
 prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                   const __grid_constant__ CUtensorMap map_v, const Params p) {
@@ -203,9 +213,10 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
   const int pos0 = ctx - q_len;
   const int rows_here = min(QT, q_len - q0);
   const int k_end = pos0 + q0 + rows_here;  // one past the last key any row of the tile reads
-  const int all_tiles = (k_end + KT - 1) / KT;
-  const int t_first = all_tiles * part / PARTS;              // this block's tiles of keys
-  const int n_tiles = all_tiles * (part + 1) / PARTS - t_first;
+  const int k_lowest = LOCAL ? first_local_key(a, pos0 + q0) : 0;  // of the tile's first row
+  const int t_lowest = k_lowest / KT, all_tiles = (k_end + KT - 1) / KT - t_lowest;
+  const int t_first = t_lowest + all_tiles * part / PARTS;   // this block's tiles of keys
+  const int n_tiles = t_lowest + all_tiles * (part + 1) / PARTS - t_first;
 
   if (threadIdx.x == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_q) : "memory");
@@ -250,7 +261,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       tma_load_2d(q_tile, &map_q, q_full, head * HD, q_start + q0);
     }
     const int* table = a.block_tables + (size_t)seq * a.table_stride;
-    const int last_page_idx = (k_end - 1) >> p.page_shift;
+    const int last_page_idx = (k_end - 1) >> p.page_shift, first_page_idx = k_lowest >> p.page_shift;
     const int boxes = KT / p.box_rows;  // 1, 2, 4 or 8
     const int group = 32 / boxes;       // tiles looked up together
     const int t_mine = lane / boxes, b_l = lane % boxes;
@@ -262,7 +273,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         const int j = (t_first + t_l) * KT + b_l * p.box_rows;
         // a box past the context re-reads the last valid page: its keys are masked anyway,
         // and what it brings is finite
-        const int pi = min(j >> p.page_shift, last_page_idx);
+        const int pi = max(min(j >> p.page_shift, last_page_idx), first_page_idx);
         const int off = (j >> p.page_shift) <= last_page_idx ? (j & (a.page_tokens - 1)) : 0;
         row_l = (table[pi] * a.num_kv_heads + kvh) * a.page_tokens + off;
       }
@@ -336,6 +347,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     float m_run = -INFINITY, l_run = 0.f;
     bool ok = true;
     const uint32_t s_col = lane_base + COL_S + st * S_COLS;
+    const int row_first = LOCAL ? first_local_key(a, qpos) : 0;
+    const int last_first = LOCAL ? first_local_key(a, k_end - 1) : 0;  // of the tile's last row
     for (int t = st, round = 0; t < n_tiles; t += 2, ++round) {
       ok = mbar_wait(&s_full[st], round & 1);
       if (!ok) break;
@@ -352,11 +365,11 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         }
       }
       const int k0 = (t_first + t) * KT;
-      if (k0 + KT - 1 > pos0 + q0) {  // keys that reach the diagonal: mask per element
+      if (k0 + KT - 1 > pos0 + q0 || (LOCAL && k0 < last_first)) {  // keys that reach an edge: mask per element
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
-          sa[j] = (k0 + j <= qpos) ? sa[j] : 0xff800000u;  // -inf
-          sb[j] = (k0 + 32 + j <= qpos) ? sb[j] : 0xff800000u;
+          sa[j] = (k0 + j <= qpos && (!LOCAL || k0 + j >= row_first)) ? sa[j] : 0xff800000u;  // -inf
+          sb[j] = (k0 + 32 + j <= qpos && (!LOCAL || k0 + 32 + j >= row_first)) ? sb[j] : 0xff800000u;
         }
       }
       // independent chains for the maximum and for the sum: a single chain of dependent
@@ -460,7 +473,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       const float mm = fmaxf(m0, m1);
       const float w0 = (m0 == -INFINITY) ? 0.f : ex2((m0 - mm) * sl2);
       const float w1 = (m1 == -INFINITY) ? 0.f : ex2((m1 - mm) * sl2);
-      const float l = pair_l[0][r] * w0 + pair_l[1][r] * w1;
+      float l = pair_l[0][r] * w0 + pair_l[1][r] * w1;
+      if (a.sinks && l > 0.f) l += ex2(a.sinks[head] * 1.4426950408889634f - mm * sl2);
       const float inv = l > 0.f ? 1.f / l : 0.f;
       const float f0 = w0 * inv, f1 = w1 * inv;
       bf16* dst = (bf16*)a.out + (size_t)(q_start + q0 + r) * a.out_row_stride + (size_t)head * HD + 32 * st;
@@ -516,6 +530,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
         o[0] = fmaf(x.x, w, o[0]); o[1] = fmaf(x.y, w, o[1]); o[2] = fmaf(x.z, w, o[2]); o[3] = fmaf(x.w, w, o[3]);
         o[4] = fmaf(y.x, w, o[4]); o[5] = fmaf(y.y, w, o[5]); o[6] = fmaf(y.z, w, o[6]); o[7] = fmaf(y.w, w, o[7]);
       }
+      if (a.sinks && l > 0.f) l += ex2(a.sinks[head] * 1.4426950408889634f - top * sl2);
       const float inv = l > 0.f ? 1.f / l : 0.f;
       uint4 w;
       w.x = pack2(o[0] * inv, o[1] * inv);
@@ -543,25 +558,25 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
 
 inline bool supported(const LseAttnArgs* a) {
   const int pt = a->page_tokens;
-  return a->dtype == LSE_BF16 && a->window == 0 && pt >= 8 && (pt & (pt - 1)) == 0 &&
+  return a->dtype == LSE_BF16 && pt >= 8 && (pt & (pt - 1)) == 0 &&
          (a->q_row_stride % 8) == 0 && (a->out_row_stride % 8) == 0;
 }
 
-template <bool CAP, int PARTS>
+template <bool CAP, int PARTS, bool LOCAL>
 inline int launch_prefill_parts(const LseAttnArgs* a, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                                 const Params& p, cudaStream_t stream) {
   constexpr int smem = Q_BYTES + 2 * STAGES * KV_BYTES + (2 * STAGES + 6) * 8 + 16 + 1024;
   static const cudaError_t configured =
-      cudaFuncSetAttribute(prefill_tc_kernel<CAP, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      cudaFuncSetAttribute(prefill_tc_kernel<CAP, PARTS, LOCAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (configured != cudaSuccess) return LSE_LAUNCH_FAILED;
   const dim3 grid(a->num_heads * PARTS, a->num_tiles);
-  return lse::launch_clusters(prefill_tc_kernel<CAP, PARTS>, grid, THREADS, PARTS, smem, stream, mq, mk, mv, p) == cudaSuccess
+  return lse::launch_clusters(prefill_tc_kernel<CAP, PARTS, LOCAL>, grid, THREADS, PARTS, smem, stream, mq, mk, mv, p) == cudaSuccess
              ? LSE_OK
              : LSE_LAUNCH_FAILED;
 }
 
 // total_rows: rows of the query tensor; pool_rows: pages * kv_heads * page_tokens.
-template <bool CAP>
+template <bool CAP, bool LOCAL>
 inline int launch_prefill_form(const LseAttnArgs* a, long long total_rows, long long pool_rows,
                           int* error_flag, cudaStream_t stream) {
   CUtensorMap mq, mk, mv;
@@ -582,19 +597,25 @@ inline int launch_prefill_form(const LseAttnArgs* a, long long total_rows, long 
   // keys 21 / 18 / 25; 128 blocks, 512 keys 16.4 / 17.4 / 29, 2000 keys 32 / 27 / 39; 144 blocks, 8184 keys 94 / 60 / 88;
   // 256 blocks, 1000 keys 23 / 29 / 51 (a further wave). The longest context is known here as what a table holds.
   const long long blocks = (long long)a->num_heads * a->num_tiles;
-  const long long keys = (long long)a->table_stride * a->page_tokens;
+  long long keys = (long long)a->table_stride * a->page_tokens;
+  if (a->window > 0) keys = keys < a->window + QT ? keys : a->window + QT;
+  if (a->chunk > 0) keys = keys < a->chunk + QT ? keys : a->chunk + QT;
   const int want = keys <= 512 || blocks > 148 ? 1 : blocks <= 32 ? 4 : 2;
   switch (want) {
-    case 1: return launch_prefill_parts<CAP, 1>(a, mq, mk, mv, p, stream);
-    case 2: return launch_prefill_parts<CAP, 2>(a, mq, mk, mv, p, stream);
-    default: return launch_prefill_parts<CAP, 4>(a, mq, mk, mv, p, stream);
+    case 1: return launch_prefill_parts<CAP, 1, LOCAL>(a, mq, mk, mv, p, stream);
+    case 2: return launch_prefill_parts<CAP, 2, LOCAL>(a, mq, mk, mv, p, stream);
+    default: return launch_prefill_parts<CAP, 4, LOCAL>(a, mq, mk, mv, p, stream);
   }
 }
 
 inline int launch_prefill(const LseAttnArgs* a, long long total_rows, long long pool_rows,
                           int* error_flag, cudaStream_t stream) {
-  return a->softcap > 0.f ? launch_prefill_form<true>(a, total_rows, pool_rows, error_flag, stream)
-                          : launch_prefill_form<false>(a, total_rows, pool_rows, error_flag, stream);
+  const bool cap = a->softcap > 0.f;
+  if (a->window > 0 || a->chunk > 0)
+    return cap ? launch_prefill_form<true, true>(a, total_rows, pool_rows, error_flag, stream)
+               : launch_prefill_form<false, true>(a, total_rows, pool_rows, error_flag, stream);
+  return cap ? launch_prefill_form<true, false>(a, total_rows, pool_rows, error_flag, stream)
+             : launch_prefill_form<false, false>(a, total_rows, pool_rows, error_flag, stream);
 }
 
 }  // namespace atc

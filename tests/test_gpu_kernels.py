@@ -390,6 +390,18 @@ def test_prefill_attention_shared_by_clusters(ops, nq, nk, q_lens, ctx_lens, pag
     ops.check_kernel_errors()
 
 
+@pytest.mark.parametrize("page", [8, 16, 64])
+@pytest.mark.parametrize("window", [1, 63, 64, 65, 130, 600, 5000])
+def test_prefill_attention_window_edges_on_tcgen05(ops, window, page):
+    """Windows that begin at, before and after a tile's edge, wider than the context, and tiles that only some rows see;
+    the tolerance of the other bfloat16 attention tests."""
+    q_lens, ctx_lens = [130, 2, 64, 257], [900, 70, 65, 257]
+    case = paged_case(4, q_lens, ctx_lens, 4, 2, 64, page, torch.bfloat16, seed=window)
+    got, ref, _ = run_attention(ops, case, 4, 2, 64, page, window, 1024)
+    close(got, ref, "bfloat16", rel16=0.02)
+    ops.check_kernel_errors()
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("window", [1, 5, 64, 100])
 def test_attention_window_edges(ops, dtype, window):
