@@ -343,7 +343,11 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
     const uint32_t lane_base = tmem + ((uint32_t)(wq * 32) << 16);
     const uint32_t o_col = lane_base + COL_O + st * O_COLS;
     const float sl2 = (CAP ? 1.f : a.scale) * 1.4426950408889634f;
-    const lse::SoftCap softcap(CAP ? a.softcap : 0.f);
+    // cap * tanh(s / cap) by tanh(y) = 1 - 2 / (1 + 2^(2 log2(e) y)); a power below the smallest number counts as zero
+    const float cap = CAP ? a.softcap : 0.f, to_exp = CAP ? a.scale * (2.8853900817779268f / a.softcap) : 0.f;
+    auto softcap = [&](uint32_t s) {
+      return __float_as_uint(fmaf(-2.f * cap, __fdividef(1.f, 1.f + ex2(__uint_as_float(s) * to_exp)), cap));
+    };
     float m_run = -INFINITY, l_run = 0.f;
     bool ok = true;
     const uint32_t s_col = lane_base + COL_S + st * S_COLS;
@@ -360,8 +364,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       if constexpr (CAP) {
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
-          sa[j] = __float_as_uint(softcap(__uint_as_float(sa[j]) * a.scale));
-          sb[j] = __float_as_uint(softcap(__uint_as_float(sb[j]) * a.scale));
+          sa[j] = softcap(sa[j]);
+          sb[j] = softcap(sb[j]);
         }
       }
       const int k0 = (t_first + t) * KT;
@@ -420,6 +424,17 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       exponentials(sb, s_col + 16);
       const float2 sum = add2(sum2[0], sum2[1]);
       l_run = sum.x + sum.y;
+      if (k0 + KT > k_end || (LOCAL && k0 < k_lowest)) {
+        // Whole tiles are copied: values beside the keys that any row sees may be anything, NaN included, and zero
+        // probabilities would not take them out. A thread of the stream clears half a row.
+        const int key = k0 + (r >> 1);
+        if (key >= k_end || key < k_lowest) {
+          uint4* row = reinterpret_cast<uint4*>(v_tiles + (t % STAGES) * KV_BYTES + (r >> 1) * (HD * 2) + (r & 1) * HD);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) row[e] = make_uint4(0, 0, 0, 0);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the multiply reads them through the async proxy
+      }
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
