@@ -5,8 +5,7 @@ available, constructing :class:`CudaOps` raises.
 
 Matrix products: float32 runs this package's own CUDA-core kernel (true 32-bit, no tensor-core
 mode). bfloat16 products of up to 32 rows (decoding) run this package's tcgen05 kernel; with more
-rows they go to cuBLAS through ``torch.mm`` with float32 accumulation, the same
-library-for-linear-layers split as the reference (src/llmserve/models/layers.py:129-152).
+rows they go to cuBLAS with float32 accumulation, the same library-for-linear-layers split as the reference (src/llmserve/models/layers.py:129-152).
 
 The few-rows kernel shares a tile's K between blocks, which add their partial sums with integer
 atomics into a buffer of 64-bit fixed-point numbers (value * 2^24). Such sums have the same bits
