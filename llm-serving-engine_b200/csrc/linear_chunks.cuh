@@ -379,8 +379,10 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_outputs_kernel(const Args a)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const float v = vs[(t + e) * LDV + tx + 16 * m];
+          // a later token's value is left out and not only met by a zero: it may be no number
+          part[b][m] = fmaf(p[b][e], t + e <= ty + 16 * b ? v : 0.f, part[b][m]);
 #pragma unroll
-          for (int i = b; i < 4; ++i) part[i][m] = fmaf(p[i][e], v, part[i][m]);
+          for (int i = b + 1; i < 4; ++i) part[i][m] = fmaf(p[i][e], v, part[i][m]);
         }
     }
 #pragma unroll

@@ -172,6 +172,24 @@ def test_linear_attention_chunk_products_at_their_edges(ops, H, dk, dv, rot, sil
     assert bool((state[[4, 6]] == 1e4).all())
 
 
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("at", [1, 15, 16, 50, 63, 64, 100])
+def test_linear_attention_chunk_products_know_nothing_of_later_tokens(ops, at, bad):
+    """A key or a value that is no number reaches no row before its token: those rows have the bits that they have
+    without it."""
+    H, dk, dv, n = 2, 64, 68, 130
+    kw = dict(num_heads=H, key_dim=dk, value_dim=dv, decay=torch.tensor([0.99, 0.5]).cuda(), activation="none",
+              key_scale=dk ** -0.5, cos=None, sin=None)
+    x = rnd(n, 2 * H * dk + H * dv, seed=3)
+    run = lambda rows: ops.decay_linear_attention(rows.cuda(), state=torch.zeros(1, H, dv, dk).cuda(),
+                                                  step=batch([n], [0], [0]), **kw).cpu()
+    clean = run(x)
+    for columns in (slice(H * dk, 2 * H * dk), slice(2 * H * dk, None), slice(0, None)):
+        dirty = x.clone()
+        dirty[at, columns] = bad
+        assert torch.equal(run(dirty)[:at], clean[:at])
+
+
 def test_linear_attention_keeps_a_key_from_far_away(ops):
     """One early key/value pair is made large; with a decay close to one it must still be most of
     the output 700 tokens later (and gone with a small decay)."""
