@@ -261,7 +261,7 @@ void gemm_bf16_library(const Tensor& a, const Tensor& w, Tensor& out, double alp
   TORCH_CHECK(status == CUBLAS_STATUS_SUCCESS, "gemm_bf16_library: the library failed with status ", num((int)status));
 }
 
-void gemm_f32(const Tensor& a, const Tensor& w, const OptTensor& bias, Tensor& out) {
+void gemm_f32(const Tensor& a, const Tensor& w, const OptTensor& bias, Tensor& out, bool w_early) {
   check_f32(a, "a");
   check_f32(w, "w");
   check_f32(out, "out");
@@ -275,7 +275,7 @@ void gemm_f32(const Tensor& a, const Tensor& w, const OptTensor& bias, Tensor& o
     b = bias->data_ptr<float>();
   }
   done(lse_gemm_f32(a.data_ptr<float>(), w.data_ptr<float>(), b, out.data_ptr<float>(),
-                    (int)a.size(0), (int)w.size(0), (int)a.size(1), stream()),
+                    (int)a.size(0), (int)w.size(0), (int)a.size(1), stream(), w_early ? 1 : 0),
        "gemm_f32");
 }
 
@@ -1446,7 +1446,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("silu_mul", &silu_mul, py::arg("gu"), py::arg("out"), py::arg("act") = 0,
         py::arg("limit") = 0.0, py::arg("col0") = 0);
   m.def("poly_norm", &poly_norm);
-  m.def("gemm_f32", &gemm_f32);
+  m.def("gemm_f32", &gemm_f32, py::arg("a"), py::arg("w"), py::arg("bias"), py::arg("out"), py::arg("w_early") = false);
   m.def("gemm_bf16_library", &gemm_bf16_library);
   m.def("gemm_bf16_skinny", &gemm_bf16_skinny);
   m.def("gemm_bf16_skinny_max_rows", &gemm_bf16_skinny_max_rows);

@@ -72,10 +72,12 @@ int lse_silu_mul(const void* gu, int in_dtype, void* out, int dtype, int T, int 
 int lse_poly_norm(const void* z, int in_dtype, const float* coef, float eps, void* out, int dtype, int T,
                   int N, cudaStream_t stream);
 
-// True float32 matrix product: out[T, N] = a[T, K] . w[N, K]^T (+ bias[N]). Each output element is
-// accumulated over k in ascending order by one thread, so a row's result does not depend on T.
+// True float32 matrix product: out[T, N] = a[T, K] . w[N, K]^T (+ bias[N]). K is cut into slices that are
+// summed by themselves and added in one order whatever T is, so a row's result does not depend on T.
+// w_early = 1: the caller knows that no kernel which may still run writes w (a model's parameter), so it may be read
+// ahead of them; with 0 both a and w may be outputs of the kernel before.
 int lse_gemm_f32(const float* a, const float* w, const float* bias, float* out, int T, int N, int K,
-                 cudaStream_t stream);
+                 cudaStream_t stream, int w_early = 0);
 
 // bfloat16 product for few rows on tcgen05 tensor cores fed by TMA (gemm_bf16_tc.cu):
 //   out[T, N] += a[T, K] . w[N, K]^T (+ bias[N]),  T <= lse_gemm_bf16_skinny_max_rows(), K % 8 == 0.

@@ -71,6 +71,8 @@ class DecoderModel:
                 raise ValueError(
                     f"{name}: got {tuple(t.shape)} {t.dtype}, want {tuple(decl.shape)} {want} contiguous"
                 )
+        # told apart from what a step computes: a product may read them before the kernels ahead of it are done
+        params = {name: torch.nn.Parameter(t, requires_grad=False) for name, t in params.items()}
         self.embed_weight = params["embed.weight"]
         self.head_weight = params["embed.weight"] if self.plan.tie_head else params["head.weight"]
         self.run_vectors = params.get("run_vectors")

@@ -301,7 +301,8 @@ class CudaOps:
             if w.dtype != torch.float32:
                 raise TypeError("float32 activations need float32 weights")
             out = torch.empty(a.shape[0], w.shape[0], dtype=torch.float32, device=a.device)
-            self.ext.gemm_f32(a, w, bias, out)
+            # a parameter of a model is no output of a kernel, so it may be read ahead of those still running
+            self.ext.gemm_f32(a, w, bias, out, type(w) is torch.nn.Parameter)
             self.launches += 1
             return out if out_dtype in (None, torch.float32) else out.to(out_dtype)
         if a.dtype != torch.bfloat16 or w.dtype != torch.bfloat16:

@@ -100,6 +100,23 @@ def test_gemm_f32_every_kernel_adds_in_the_same_order(ops, N, K):
         assert torch.equal(run(a[first : first + n]), whole[first : first + n]), (first, n)
 
 
+@pytest.mark.parametrize("T", [1, 9, 40])
+def test_gemm_f32_with_weights_of_the_kernel_before(ops, T):
+    """Both operands may be what a kernel of this package, launched just before, still writes; a parameter, which is
+    read ahead of it, gives the same bits."""
+    N, K = 4096, 1024
+    x, a, scale = rnd(N, K, seed=1).cuda(), rnd(T, K, seed=2).cuda(), torch.ones(K).cuda()
+    for i in range(20):
+        x = x.flip(0).contiguous()
+        w = ops.add_rmsnorm(x, None, scale, 1e-6, torch.float32)
+        got = ops.linear(a, w, None, out_dtype=torch.float32)
+        torch.cuda.synchronize()
+        assert torch.equal(got, ops.linear(a, w.clone(), None, out_dtype=torch.float32)), i
+        assert torch.equal(got, ops.linear(a, torch.nn.Parameter(w.clone(), requires_grad=False), None, out_dtype=torch.float32))
+        w.fill_(float("nan"))  # the next one gets this memory
+        del w
+
+
 @pytest.mark.parametrize("T,N,K", [(1, 48, 64), (9, 520, 200), (16, 128, 64), (17, 2048, 2048),
                                    (8, 16384, 2048), (4, 49152, 2048), (8, 6144, 2048), (2, 2048, 8192),
                                    (64, 136, 1000), (100, 384, 8192), (256, 1000, 520), (300, 136, 1000)])
