@@ -3,6 +3,7 @@
 // PyTorch's current CUDA stream. Attention kernels live in one shared library per head size,
 // loaded here with dlopen.
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/tunable/Tunable.h>
 #include <cublas_v2.h>
 #include <dlfcn.h>
 #include <torch/extension.h>
@@ -238,19 +239,24 @@ void poly_norm(const Tensor& z, const Tensor& coef, double eps, Tensor& out) {
 }
 
 // out = alpha a w^T (+ out) by the library, float32 sums, as torch.mm and torch.addmm call it by default: the same
-// function with the same arguments, without the views, the argument parsing and the dispatch in front of it.
-void gemm_bf16_library(const Tensor& a, const Tensor& w, Tensor& out, double alpha, bool accumulate) {
-  for (const Tensor* t : {&a, &w}) {
-    TORCH_CHECK(t->is_cuda() && t->is_contiguous() && t->dim() == 2 && t->scalar_type() == torch::kBFloat16,
-                "gemm_bf16_library: a and w must be contiguous bfloat16 CUDA matrices");
-  }
-  TORCH_CHECK(out.is_cuda() && out.is_contiguous() && out.dim() == 2, "gemm_bf16_library: out must be a contiguous CUDA matrix");
+// function with the same arguments, without the views, the argument parsing and the dispatch in front of it. false:
+// torch's own call has to serve this one (nothing was done) -- empty or other than plain matrices, matrices of another
+// device than the current one, gradients, or any setting of torch's that changes which function it calls or how.
+bool gemm_bf16_library(const Tensor& a, const Tensor& w, Tensor& out, double alpha, bool accumulate) {
+  for (const Tensor* t : {&a, &w, static_cast<const Tensor*>(&out)})
+    if (!t->is_cuda() || !t->is_contiguous() || t->dim() != 2 || t->device().index() != at::cuda::current_device()) return false;
   const int64_t T = a.size(0), N = w.size(0), K = a.size(1);
-  TORCH_CHECK(T > 0 && N > 0 && K > 0 && w.size(1) == K && out.size(0) == T && out.size(1) == N,
-              "gemm_bf16_library: need a [T, K], w [N, K], out [T, N]");
-  TORCH_CHECK(out.scalar_type() == torch::kBFloat16 || out.scalar_type() == torch::kFloat32,
-              "gemm_bf16_library: out must be bfloat16 or float32");
-  TORCH_CHECK(std::max({T, N, K}) <= INT_MAX, "gemm_bf16_library: sizes beyond 32 bits");
+  if (a.scalar_type() != torch::kBFloat16 || w.scalar_type() != torch::kBFloat16 ||
+      (out.scalar_type() != torch::kBFloat16 && out.scalar_type() != torch::kFloat32) || T <= 0 || N <= 0 || K <= 0 ||
+      w.size(1) != K || out.size(0) != T || out.size(1) != N || std::max({T, N, K}) > INT_MAX)
+    return false;
+  const auto& context = at::globalContext();
+  if (context.allowBF16ReductionCuBLAS() != at::CuBLASReductionOption::AllowReducedPrecisionWithSplitK ||
+      context.deterministicAlgorithms() || at::cuda::tunable::getTuningContext()->IsTunableOpEnabled())
+    return false;
+  const at::BlasBackend backend = at::globalContext().blasPreferredBackend();
+  if (backend != at::BlasBackend::Default && backend != at::BlasBackend::Cublas) return false;
+  if (at::GradMode::is_enabled() && (a.requires_grad() || w.requires_grad() || out.requires_grad())) return false;
   const float one = (float)alpha, beta = accumulate ? 1.f : 0.f;
   cublasHandle_t handle = at::cuda::getCurrentCUDABlasHandle();  // on the current stream, with torch's workspace
   const cublasStatus_t status =
@@ -259,6 +265,7 @@ void gemm_bf16_library(const Tensor& a, const Tensor& w, Tensor& out, double alp
                    out.scalar_type() == torch::kFloat32 ? CUDA_R_32F : CUDA_R_16BF, (int)N, CUBLAS_COMPUTE_32F,
                    CUBLAS_GEMM_DEFAULT_TENSOR_OP);
   TORCH_CHECK(status == CUBLAS_STATUS_SUCCESS, "gemm_bf16_library: the library failed with status ", num((int)status));
+  return true;
 }
 
 void gemm_f32(const Tensor& a, const Tensor& w, const OptTensor& bias, Tensor& out, bool w_early) {

@@ -323,21 +323,19 @@ class CudaOps:
             self.launches += 1
             self._sums_taken(sums)
             return out
-        # many rows: the library. Called from the binding where nothing has to be arranged first: torch's own call
-        # of it costs 11 us of the host (with the view of w), this one 5, four times a layer.
-        # (A caller who has forbidden torch's reduced-precision sums, or allowed it to accumulate otherwise, gets
-        # torch's call.)
-        plain = (bias is None and T > 0 and a.is_contiguous() and w.is_contiguous()
-                 and torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction is True)
+        # many rows: the library. Called from the binding where torch has nothing to arrange: torch's own call of it
+        # costs 11 us of the host (with the view of w), this one 5, four times a layer. The binding leaves to torch
+        # what it would call otherwise (empty matrices, another library preferred, ...).
         into = accumulate_into
-        if plain and into is not None and into.dtype == torch.float32 and into.is_contiguous():
+        if bias is None and into is not None:
             # added into the residual stream (beta = 1)
-            self.ext.gemm_bf16_library(a, w, into, 1.0 if coefficient is None else float(coefficient), True)
-            return None
-        if plain and out_dtype in (None, torch.bfloat16, torch.float32):
+            if into.dtype == torch.float32 and self.ext.gemm_bf16_library(
+                    a, w, into, 1.0 if coefficient is None else float(coefficient), True):
+                return None
+        elif bias is None and out_dtype in (None, torch.bfloat16, torch.float32):
             out = torch.empty(T, N, dtype=out_dtype or torch.bfloat16, device=a.device)
-            self.ext.gemm_bf16_library(a, w, out, 1.0, False)
-            return out
+            if self.ext.gemm_bf16_library(a, w, out, 1.0, False):
+                return out
         if accumulate_into is not None and bias is None and self._addmm_in_place is not False:
             try:
                 torch.addmm(accumulate_into, a, w.t(), out_dtype=torch.float32, out=accumulate_into,

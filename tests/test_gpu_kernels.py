@@ -419,6 +419,44 @@ def test_prefill_attention_window_edges_on_tcgen05(ops, window, page):
     ops.check_kernel_errors()
 
 
+@pytest.mark.parametrize("T,N,K", [(40, 0, 64), (40, 24, 0), (40, 24, 64)])
+def test_library_product_takes_what_torch_takes(ops, T, N, K):
+    """No features, no terms, a result that is added into a matrix with other strides: as torch.mm and torch.addmm."""
+    a, w = rnd(T, K, seed=1).bfloat16().cuda(), rnd(N, K, seed=2).bfloat16().cuda()
+    for out_dtype in (None, torch.float32):
+        got = ops.linear(a, w, None, out_dtype=out_dtype)
+        assert got.dtype == (out_dtype or torch.bfloat16) and torch.equal(got, torch.mm(a, w.t(), out_dtype=got.dtype))
+    for into in (rnd(T, N, seed=3).cuda(), rnd(N, T, seed=3).cuda().t()):
+        want = into + 0.5 * torch.mm(a, w.t(), out_dtype=torch.float32)
+        y = ops.linear(a, w, None, out_dtype=torch.float32, accumulate_into=into, coefficient=0.5)
+        got = into if y is None else into + 0.5 * y
+        # one fused add where torch rounds twice
+        assert y is None and torch.allclose(got, want, rtol=2.0**-22, atol=2.0**-22 * 64)
+
+
+def test_library_product_follows_torchs_settings(ops, monkeypatch):
+    """Where a setting of torch's changes what it calls, torch makes the call."""
+    a, w = rnd(40, 64, seed=1).bfloat16().cuda(), rnd(24, 64, seed=2).bfloat16().cuda()
+    calls, mm = [], torch.mm
+    monkeypatch.setattr(torch, "mm", lambda *x, **k: calls.append(1) or mm(*x, **k))
+    ops.linear(a, w)
+    assert not calls
+    before = torch.backends.cuda.preferred_blas_library()
+    try:
+        torch.backends.cuda.preferred_blas_library("cublaslt")
+        ops.linear(a, w)
+    finally:
+        torch.backends.cuda.preferred_blas_library(before)
+    assert len(calls) == 1
+    try:
+        torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = False
+        ops.linear(a, w)
+    finally:
+        torch.backends.cuda.matmul.allow_bf16_reduced_precision_reduction = True
+    assert len(calls) == 2
+    assert ops.linear(a.requires_grad_(), w).requires_grad and len(calls) == 3
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("window", [1, 5, 64, 100])
 def test_attention_window_edges(ops, dtype, window):
