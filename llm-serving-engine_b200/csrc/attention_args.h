@@ -75,6 +75,9 @@ struct LseAttnArgs {
   //   softcap > 0: the scaled score s becomes softcap * tanh(s / softcap) (before the distance penalty).
   //   Every kernel serves it, except single tokens straight from qkv_sums.
   float softcap;
+  // Longest context among the portions (lse_attn_prefill) where the caller knows a bound; 0: what a row of the
+  // block tables holds. It decides how blocks share the work and never what is computed.
+  int max_portion_ctx;
 };
 
 #define LSE_ATTN_COUNTERS 65536  // words at the start of the scratch: one counter per (sequence, head group)

@@ -607,15 +607,23 @@ inline int launch_prefill_form(const LseAttnArgs* a, long long total_rows, long 
   while ((1 << p.page_shift) < a->page_tokens) ++p.page_shift;
   p.error_flag = error_flag;
   // Two blocks run on an SM at a time. A grid that leaves half of these places empty is as slow as its longest block,
-  // so the keys of a (query tile, head) are shared by a cluster. Measured alone, 1 / 2 / 4 blocks each, us:
-  // 9 blocks, 512 keys 16.4 / 14.6 / 14.5, 4000 keys 51 / 33 / 25; 32 blocks, 2048 keys 31 / 23 / 21; 72 blocks, 1024
-  // keys 21 / 18 / 25; 128 blocks, 512 keys 16.4 / 17.4 / 29, 2000 keys 32 / 27 / 39; 144 blocks, 8184 keys 94 / 60 / 88;
-  // 256 blocks, 1000 keys 23 / 29 / 51 (a further wave). The longest context is known here as what a table holds.
+  // so the keys of a (query tile, head) are shared by a cluster where they are enough to pay for its barriers and
+  // merge. Back to back, 1 / 2 / 4 blocks each, us: 9 blocks, 40 keys 10.3 / 12.3 / 14.3 (alone), 512 keys
+  // 10.1 / 9.0 / 8.8, 768 keys 12.7 / 10.4 / 9.3, 4096 keys 46 / 27 / 18; 32 blocks, 640 keys 11.0 / 11.7 / 12.3, 768 keys
+  // 12.3 / 12.2 / 12.4, 1024 keys 14.8 / 13.9 / 13.2, 4096 keys 46 / 31 / 23; 64 blocks, 512 keys 10.9 / 11.8 / 13.0, 640 keys
+  // 12.4 / 12.7 / 13.1 in one portion and 13.4 / 12.7 / 13.4 in four; 128 blocks, 640 keys 12.7 / 13.0 / 23 and
+  // 14.1 / 13.4 / 26, 1024 keys 17.8 / 15.6 / 26, 4096 keys 56 / 36 / 46; 256 blocks, 1000 keys 23 / 29 / 51 (alone; a
+  // further wave).
   const long long blocks = (long long)a->num_heads * a->num_tiles;
   long long keys = (long long)a->table_stride * a->page_tokens;
-  if (a->window > 0) keys = keys < a->window + QT ? keys : a->window + QT;
-  if (a->chunk > 0) keys = keys < a->chunk + QT ? keys : a->chunk + QT;
-  const int want = keys <= 512 || blocks > 148 ? 1 : blocks <= 32 ? 4 : 2;
+  auto at_most = [&](long long n) { keys = keys < n ? keys : n; };
+  if (a->max_portion_ctx > 0) at_most(a->max_portion_ctx);
+  if (a->window > 0) at_most((long long)a->window + QT);
+  if (a->chunk > 0) at_most((long long)a->chunk + QT);
+  int want = 1;
+  if (blocks <= 18) want = keys > 512 ? 4 : 1;
+  else if (blocks <= 32) want = keys >= 1024 ? 4 : keys >= 768 ? 2 : 1;
+  else if (blocks <= 148) want = keys >= 640 ? 2 : 1;
   switch (want) {
     case 1: return launch_prefill_parts<CAP, 1, LOCAL>(a, mq, mk, mv, p, stream);
     case 2: return launch_prefill_parts<CAP, 2, LOCAL>(a, mq, mk, mv, p, stream);

@@ -402,7 +402,7 @@ void paged_attention(const Tensor& q, Tensor& out, const Tensor& k_pages, const 
                      const OptTensor& decode_seqs, int64_t num_decode, int64_t num_splits,
                      const OptTensor& scratch, int64_t force_kernel, const OptTensor& head_scale,
                      const OptTensor& slopes, int64_t chunk, const OptTensor& sinks, int64_t keep_first,
-                     double softcap) {
+                     double softcap, int64_t max_portion_ctx) {
   const AttnLib& lib = attn_lib(D);
   TORCH_CHECK(q.is_cuda() && q.dim() == 2 && q.stride(1) == 1 && q.size(1) >= num_heads * D,
               "paged_attention: q must be [T, >= heads*head_dim] with unit column stride");
@@ -466,6 +466,7 @@ void paged_attention(const Tensor& q, Tensor& out, const Tensor& k_pages, const 
   a.keep_first = (int)keep_first;
   TORCH_CHECK(softcap >= 0, "paged_attention: softcap must not be negative");
   a.softcap = (float)softcap;
+  a.max_portion_ctx = (int)max_portion_ctx;
   if (sinks) {
     check_f32(*sinks, "sinks");
     TORCH_CHECK(sinks->numel() == num_heads, "paged_attention: sinks needs one value per head");
@@ -1469,7 +1470,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("block_tables"), py::arg("ctx_lens"), py::arg("cu_q"), py::arg("tiles"), py::arg("num_tiles"),
         py::arg("decode_seqs"), py::arg("num_decode"), py::arg("num_splits"), py::arg("scratch"),
         py::arg("force_kernel"), py::arg("head_scale"), py::arg("slopes"), py::arg("chunk"),
-        py::arg("sinks") = py::none(), py::arg("keep_first") = 0, py::arg("softcap") = 0.0);
+        py::arg("sinks") = py::none(), py::arg("keep_first") = 0, py::arg("softcap") = 0.0, py::arg("max_portion_ctx") = 0);
   m.def("hashed_pair_add", &hashed_pair_add);
   m.def("sinusoid_add", &sinusoid_add);
   m.def("latent_write", &latent_write);

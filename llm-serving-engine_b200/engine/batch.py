@@ -67,6 +67,7 @@ class DeviceStep:
     decode_splits: int  # fixed number of context partitions, or 0 to let the kernels choose
     plans: dict[Any, dict[str, Any]]
     host: HostStep | None = None
+    max_portion_ctx: int = 0  # bound of the contexts of the sequences with more than one token (0: not known)
     every_row_wanted: bool = False  # logit_rows is 0, 1, ..., num_tokens - 1: the final norm need not gather
 
 

@@ -137,7 +137,7 @@ class _MixedGraph:
     they give the lists' names and shapes."""
 
     def __init__(self, owner: "DecodeGraphs", batch: int, slots: int, tokens: int, splits: int,
-                 sampled: bool, kinds: int, plans: dict) -> None:
+                 sampled: bool, kinds: int, plans: dict, max_portion_ctx: int = 0) -> None:
         runner = owner.runner
         dev = runner.device
         self.batch, self.slots, self.pre_tokens = batch, slots, tokens
@@ -167,7 +167,7 @@ class _MixedGraph:
             first_portion=view("first_portion"),
             block_tables=[view(("table", gi)).view(N, -1) for gi in range(len(runner.manager.groups))],
             logit_rows=view("logit_rows"), num_tokens=T, num_seqs=N, num_logit_rows=N,
-            max_decode_ctx=0, decode_splits=splits,
+            max_decode_ctx=0, decode_splits=splits, max_portion_ctx=max_portion_ctx,
             plans={key: {name: view(("plan", key, name)).view(a.shape) for name, a in plan.items()}
                    for key, plan in plans.items()},
             host=None,
@@ -452,10 +452,12 @@ class DecodeGraphs:
         splits = runner.ops.decode_splits(B, self.min_kv_heads, max_ctx, runner.dtype) if B else 1
         # unsampled and padding rows are greedy, so the one-block kernel is always there
         kinds = (sample_kinds(r.params for r in rows) | 1) if simple else 0
-        key = (B, P, TP, splits, simple, kinds)
+        # how blocks share a portion's keys is captured too: short contexts have a graph of their own
+        longest = runner.ops.portion_ctx_bound(int(arrays["ctx_lens"][B:].max()), runner.dtype)
+        key = (B, P, TP, splits, simple, kinds, longest)
         g = self.graphs.get(key)
         if g is None:
-            g = self.graphs[key] = _MixedGraph(self, B, P, TP, splits, simple, kinds, plans)
+            g = self.graphs[key] = _MixedGraph(self, B, P, TP, splits, simple, kinds, plans, longest)
         if g.h2d_done is not None:
             g.h2d_done.synchronize()
         for name, a in arrays.items():

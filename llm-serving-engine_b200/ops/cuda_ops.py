@@ -465,6 +465,12 @@ class CudaOps:
         return choose_decode_splits(num_decode * num_kv_heads, max_ctx, self.num_sms, self.decode_blocks_per_sm,
                                     32 if dtype == torch.float32 else 128)
 
+    def portion_ctx_bound(self, max_ctx: int, dtype: torch.dtype) -> int:
+        """What a captured step knows of its portions' contexts: a bound of them, or 0 for any length. Two values
+        only (a step is captured for each), and one where no kernel looks at it: the tcgen05 kernel (bfloat16, head
+        size 64) never shares up to 512 keys between blocks."""
+        return 512 if max_ctx <= 512 and dtype == torch.bfloat16 and 64 in self._attn_loaded else 0
+
     def paged_attention(self, q, *, num_heads, num_kv_heads, head_dim, scale, window, k_pages,
                         v_pages, block_tables, page_tokens, step, plan, head_scale=None, slopes=None,
                         chunk=0, sinks=None, keep_first=0, out_dtype=None, softcap=0.0):
@@ -489,7 +495,7 @@ class CudaOps:
             plan["tiles"] if n_tiles else None, n_tiles,
             plan["decode_seqs"] if n_dec else None, n_dec, splits, scratch,
             self.attention_kernel, head_scale, slopes, int(chunk), sinks, int(keep_first) if window else 0,
-            float(softcap),
+            float(softcap), int(getattr(step, "max_portion_ctx", 0)),
         )
         self.launches += (1 if n_tiles else 0) + (1 if n_dec else 0)
         return out

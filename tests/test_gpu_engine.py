@@ -144,6 +144,26 @@ def test_captured_steps_with_portions_give_the_same_tokens(sharp_dirs, name, dty
                     assert_same_or_near_tie(sharp_dirs[name], prompts[k], a, b)
 
 
+def test_captured_portions_know_whether_their_contexts_are_short(sharp_dirs):
+    """The same shapes early and late in long prompts are captured apart (head size 64, bfloat16): the blocks of a step
+    share a portion's keys or do not. Same tokens as kernel by kernel."""
+    import numpy as np
+
+    rng = np.random.default_rng(8)
+    prompts = [rng.integers(0, TINY["C"]["vocab_size"], n).tolist() for n in (70, 720, 40)]
+    runs = {}
+    for graphs in (False, True):
+        m = llm(sharp_dirs["C"], "C", "bfloat16", cuda_graphs=graphs, max_num_batched_tokens=64, num_kv_blocks=200)
+        if graphs:
+            m.engine.runner._graphs().capture_after = 1
+        runs[graphs] = [o.outputs[0].token_ids for o in m.generate(prompts, [greedy(6)] * 3)]
+        if graphs:
+            held = m.engine.runner.decode_graphs.graphs.values()
+            assert {g.step.max_portion_ctx for g in held if g.slots > 0 and g.graph is not None} == {0, 512}
+    for p, a, b in zip(prompts, runs[True], runs[False], strict=True):
+        assert_same_or_near_tie(sharp_dirs["C"], p, a, b)
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_random_arrivals_give_the_same_tokens_with_and_without_graphs(sharp_dirs, dtype):
     """Requests of every sampling kind arrive at random moments into a cache so small that some are

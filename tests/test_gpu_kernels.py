@@ -407,6 +407,23 @@ def test_prefill_attention_shared_by_clusters(ops, nq, nk, q_lens, ctx_lens, pag
     ops.check_kernel_errors()
 
 
+@pytest.mark.parametrize("nq,nk,q_lens,ctx_lens", [(2, 1, [100], [300]), (24, 8, [129, 2, 128], [500, 2, 449])])
+def test_prefill_attention_of_short_contexts_under_wide_tables(ops, nq, nk, q_lens, ctx_lens):
+    """Block tables as wide as the longest request allowed, as captured steps have them: with the contexts' bound known
+    the portions run as under tables of their own width, bit for bit."""
+    qkv, kp, vp, tables, *_, step = paged_case(len(q_lens), q_lens, ctx_lens, nq, nk, 64, 16, torch.bfloat16, seed=nq)
+    ops.check_attention_shape(64, torch.bfloat16)
+    plan = {k: torch.from_numpy(v).cuda() for k, v in ops.attention_plan(step, torch.bfloat16, 64).items()}
+    kw = dict(num_heads=nq, num_kv_heads=nk, head_dim=64, scale=0.125, window=0, k_pages=kp.cuda(), v_pages=vp.cuda(),
+              page_tokens=16, plan=plan)
+    run = lambda t, bound: ops.paged_attention(qkv.cuda()[:, : nq * 64], block_tables=t.cuda(), step=SimpleNamespace(
+        cu_q=step.cu_q.cuda(), ctx_lens=step.ctx_lens.cuda(), decode_splits=0, max_decode_ctx=0, max_portion_ctx=bound), **kw)
+    wide = torch.cat([tables, torch.zeros(len(q_lens), 200, dtype=torch.int32)], 1)
+    bound = ops.portion_ctx_bound(max(ctx_lens), torch.bfloat16)
+    assert bound >= max(ctx_lens) and ops.portion_ctx_bound(513, torch.bfloat16) == 0
+    assert torch.equal(run(wide, bound), run(tables, 0))
+
+
 @pytest.mark.parametrize("page", [8, 16, 64])
 @pytest.mark.parametrize("window", [1, 63, 64, 65, 130, 600, 5000])
 def test_prefill_attention_window_edges_on_tcgen05(ops, window, page):
