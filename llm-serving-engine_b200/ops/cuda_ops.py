@@ -100,9 +100,9 @@ def choose_decode_splits(pairs: int, max_ctx: int, num_sms: int, blocks_per_sm: 
     24 sequences took 79. So the number of partitions is the one that minimises
     ``waves * (keys per block + a block's fixed cost)``, among partitions of ``min_keys`` keys or more
     (128: measured at one sequence of 2176 keys: 8 partitions 13.3 us, 16 10.9, 28 11.9, 34 12.1).
-    The context is rounded up to a power of two first, so that the choice (which captured graphs
-    are keyed on) does not flicker from step to step. Without a known occupancy: about six blocks
-    per SM.
+    The context is rounded up to a power of two for the cost, so that the choice (which captured
+    graphs are keyed on) seldom changes from step to step; how many partitions of ``min_keys`` there
+    can be follows the context itself. Without a known occupancy: about six blocks per SM.
     """
     if pairs <= 0:
         return 1
@@ -134,6 +134,7 @@ class CudaOps:
         self._attn_loaded: set[int] = set()
         self._scratch: torch.Tensor | None = None
         self.decode_blocks_per_sm = 0  # of the single-token attention kernel; 0: not asked yet
+        self.decode_group = 0  # query heads per key head, the least of the layers asked about; 0: not asked yet
         self.fuse_rotation_into_attention = True  # single tokens: attention makes q, k, v from the product's sums
         self._takes_sums_known: dict[tuple, bool] = {}
         self._sample_scratch: torch.Tensor | None = None
@@ -172,6 +173,8 @@ class CudaOps:
                                                             num_heads, num_kv_heads))
             if n > 0:
                 self.decode_blocks_per_sm = min(self.decode_blocks_per_sm or n, n)
+            group = num_heads // num_kv_heads
+            self.decode_group = min(self.decode_group or group, group)
 
     def reserve_attention_scratch(self, head_dim: int, max_decode: int, num_heads: int,
                                   max_splits: int = 64) -> None:
@@ -461,9 +464,18 @@ class CudaOps:
     def decode_splits(self, num_decode, num_kv_heads, max_ctx, dtype=None):
         """Context partitions per (sequence, head) for a step of single tokens. The float32 kernel has 16 keys of a
         block in flight where the bfloat16 one has 64, so its partitions may be shorter: 6 sequences of 300 keys, 9
-        heads on 3 key heads, 24 steps of 30 layers in partitions of 128 / 64 / 32 / 16 keys 55.2 / 52.5 / 51.5 / 51.3 ms."""
-        return choose_decode_splits(num_decode * num_kv_heads, max_ctx, self.num_sms, self.decode_blocks_per_sm,
-                                    32 if dtype == torch.float32 else 128)
+        heads on 3 key heads, 24 steps of 30 layers in partitions of 128 / 64 / 32 / 16 keys 55.2 / 52.5 / 51.5 / 51.3 ms.
+        There the power of two above the context also bounds how many they are: one choice (and one captured graph)
+        per doubling. Contexts that a block walks faster than partitions are merged stay whole: up to 64 keys (one
+        sequence of 33 keys, 9 heads on 3: whole 6.0 us, in two 7.2; of 100 keys: 10.0, in four 8.0), up to 128 where
+        a key head serves one query head (one sequence of 100 keys, 32 heads: 5.6, in four 5.7; six: 7.0, in three
+        7.5; one of 200: in two 8.0, in eight 6.9)."""
+        pairs, min_keys = num_decode * num_kv_heads, 128
+        if dtype == torch.float32:
+            max_ctx, min_keys = 1 << max(0, int(max_ctx) - 1).bit_length(), 32
+            if max_ctx <= (128 if self.decode_group == 1 else 64):
+                return 1
+        return choose_decode_splits(pairs, max_ctx, self.num_sms, self.decode_blocks_per_sm, min_keys)
 
     def portion_ctx_bound(self, max_ctx: int, dtype: torch.dtype) -> int:
         """What a captured step knows of its portions' contexts: a bound of them, or 0 for any length. Two values

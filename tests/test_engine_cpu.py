@@ -368,6 +368,28 @@ def test_a_kernel_that_gave_up_waiting_stops_the_engine(sharp_dirs):
         eng.step()
 
 
+@pytest.mark.parametrize("group,blocks_per_sm", [(1, 8), (1, 0), (3, 5), (3, 0), (4, 6)])
+def test_float32_context_partitions_change_once_per_doubling(group, blocks_per_sm):
+    """Captured graphs are keyed on the number of partitions. For float32 it is one number from one power of two to the
+    next, at most 64 (what the scratch is reserved for), of 16 keys or more each; short contexts stay whole."""
+    import torch
+
+    from llmserve_b200.ops.cuda_ops import CudaOps
+
+    ops = CudaOps.__new__(CudaOps)
+    ops.num_sms, ops.decode_blocks_per_sm, ops.decode_group = 148, blocks_per_sm, group
+    for batch in (1, 2, 6, 8, 24, 64):
+        pick = lambda ctx: ops.decode_splits(batch, 3, ctx, torch.float32)
+        last = 1
+        for top in (32, 64, 128, 256, 512, 1024, 2048, 4096, 8192, 16384):
+            got = {pick(ctx) for ctx in range(last, top + 1, max(1, (top - last) // 64))} | {pick(top)}
+            assert len(got) == 1
+            s = got.pop()
+            assert 1 <= s <= 64 and (s == 1 or last // s >= 16)
+            assert s == 1 or top > (128 if group == 1 else 64)
+            last = top + 1
+
+
 def test_context_partitions_fill_whole_waves():
     """148 SMs holding 7 blocks each run 1036 blocks at a time. The number of partitions per
     (sequence, head) avoids a last wave that is nearly empty, keeps partitions of 128 keys or
