@@ -13,9 +13,12 @@
 //              streaming w once; measured it is the latency of a block (load, multiply, 32 partial sums), with
 //              two blocks of 110 KB per SM. 6 rows, K = 576: 49152 features 64 us (w at copy rate: 17), 3072
 //              features 12 us; 576 features of K = 1536 12 us (all with 6 us of start and timing);
-//   tiles      BM x BN outputs per block, 4 x 4 per thread, the next K tile on its way in registers
-//              while this one is multiplied: bound by the FMA units. Where 64 x 64 tiles would leave
-//              SMs idle, 32 x 32 tiles whose four groups of K are summed by four sets of threads.
+//   tiles      BM x BN outputs per block, TM x 4 per thread, the next K tile on its way in registers
+//              while this one is multiplied: bound by the reads of shared memory (64 x 128 tiles of 8 x 4 per
+//              thread: 900 rows of 49152 x 576 in 1388 us, 37 TFLOP/s; 64 x 64 of 4 x 4: 1613). Where these
+//              would leave SMs idle, 32 x 32 tiles whose four groups of K are summed by four sets of threads.
+#include <climits>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -66,12 +69,9 @@ __global__ void __launch_bounds__(32 * NG) few_rows_kernel(const Args p) {
   };
   // Where the caller says that w depends on no kernel still running, its first passes are asked for before the wait:
   // 24 steps of 6 rows, 30 layers, 41.7 ms against 44.1 after it (prefetching them into L2 instead: 44.0).
-  auto first_weights = [&]() {
-    for (int c = 0; c < STAGES - 1 && c < passes; ++c) load(c, NB, 0, p.w, n0, p.N);
-  };
-  if (p.w_early) first_weights();
-  pdl_wait();
-  if (!p.w_early) first_weights();
+  if (!p.w_early) pdl_wait();
+  for (int c = 0; c < STAGES - 1 && c < passes; ++c) load(c, NB, 0, p.w, n0, p.N);
+  if (p.w_early) pdl_wait();
   for (int c = 0; c < STAGES - 1; ++c) {
     if (c < passes) load(c, FEW_T, NB, p.a, t0, p.T);
     asm volatile("cp.async.commit_group;\n" ::);
@@ -133,30 +133,35 @@ __global__ void __launch_bounds__(32 * NG) few_rows_kernel(const Args p) {
 }
 
 // ---------------------------------------------------------------------------------------- tiles
-// G sets of threads; set g sums the groups of slices g * 4 / G .. of K (G = 1: all of them).
+// G = 4: four sets of threads, set g sums group g of the slices. G = 1: one set sums all of K; the sum of the groups
+// so far lies in shared memory, where it is touched four times in all: in registers it cost a block per SM (64 x 64
+// tiles, 900 rows, 3072 x 576: 125 us; now 113, as the single chain of additions took before there were slices, 111).
 constexpr int BK = 16;
 
-template <int BM, int BN, int G>
-__global__ void __launch_bounds__(G * (BM / 4) * (BN / 4)) tiles_kernel(const Args p, const bool vec) {
-  constexpr int SET = (BM / 4) * (BN / 4);              // threads of a set
+template <int BM, int BN, int TM, int G, int BLOCKS>
+__global__ void __launch_bounds__(G * (BM / TM) * (BN / 4), BLOCKS) tiles_kernel(const Args p, const bool vec) {
+  constexpr int SET = (BM / TM) * (BN / 4);             // threads of a set
   constexpr int PA = BM * 4 / SET, PW = BN * 4 / SET;   // pieces of four k per thread and tile
   static_assert(BM * 4 % SET == 0 && BN * 4 % SET == 0, "");
   constexpr int LA = BM + 4, LW = BN + 4, TILE = BK * (LA + LW);
-  __shared__ __align__(16) float smem[G * 2 * TILE];
+  extern __shared__ __align__(16) float smem[];  // the sets' tiles, two each; G == 1: then the totals
   static_assert(G == 1 || G * BM * BN <= G * 2 * TILE, "");
   pdl_trigger();
   const int set = threadIdx.x / SET, tid = threadIdx.x % SET;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  const int tm = (tid / (BN / 4)) * 4, tn = (tid % (BN / 4)) * 4;
+  const int tm = (tid / (BN / 4)) * TM, tn = (tid % (BN / 4)) * 4;
   float* tiles = smem + set * 2 * TILE;
+  float4* mine = reinterpret_cast<float4*>(smem + G * 2 * TILE) + tid;  // [TM][SET]
   const int per_set = SLICES / G * p.SL;                // elements of K per set, a multiple of BK
   const int k_begin = set * per_set;
   const int n_tiles = ((G == 1 ? p.K : min(p.K, per_set)) + BK - 1) / BK;  // the same for every set
-  float acc[4][4], grp[4][4], tot[4][4];
+  float acc[TM][4], grp[TM][4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < TM; ++i) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = grp[i][j] = tot[i][j] = 0.f;
+    for (int j = 0; j < 4; ++j) acc[i][j] = grp[i][j] = 0.f;
+    if (G == 1) mine[i * SET] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
   float4 av[PA], wv[PW];
   auto piece = [&](const float* src, int row, int limit, int k) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -202,14 +207,24 @@ __global__ void __launch_bounds__(G * (BM / 4) * (BN / 4)) tiles_kernel(const Ar
       ws[(k + 2) * LW + r] = wv[i].z; ws[(k + 3) * LW + r] = wv[i].w;
     }
   };
-  auto add_into = [](float (&to)[4][4], float (&from)[4][4]) {
+  auto end_of_slice = [&]() {
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < TM; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        to[i][j] += from[i][j];
-        from[i][j] = 0.f;
+        grp[i][j] += acc[i][j];
+        acc[i][j] = 0.f;
       }
+  };
+  auto end_of_group = [&]() {  // G == 1
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+      float4 t = mine[i * SET];
+      t.x += grp[i][0]; t.y += grp[i][1]; t.z += grp[i][2]; t.w += grp[i][3];
+      mine[i * SET] = t;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) grp[i][j] = 0.f;
+    }
   };
   pdl_wait();
   fetch(0);
@@ -224,34 +239,37 @@ __global__ void __launch_bounds__(G * (BM / 4) * (BN / 4)) tiles_kernel(const Ar
     for (int half = 0; half < 2; ++half) {
 #pragma unroll
       for (int kk = 8 * half; kk < 8 * half + 8; ++kk) {
-        const float4 x = *reinterpret_cast<const float4*>(as + kk * LA);
         const float4 y = *reinterpret_cast<const float4*>(ws + kk * LW);
-        const float xr[4] = {x.x, x.y, x.z, x.w}, yr[4] = {y.x, y.y, y.z, y.w};
+        const float yr[4] = {y.x, y.y, y.z, y.w};
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int q = 0; q < TM / 4; ++q) {
+          const float4 x = *reinterpret_cast<const float4*>(as + kk * LA + 4 * q);
+          const float xr[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-          for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(xr[i], yr[j], acc[i][j]);
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[4 * q + i][j] = fmaf(xr[i], yr[j], acc[4 * q + i][j]);
+        }
       }
       left -= 8;
-      if (left == 0) {  // the end of a slice
+      if (left == 0) {
         left = p.SL;
-        add_into(grp, acc);
+        end_of_slice();
         if (--slices == 0) {
           slices = GROUP;
-          if (G == 1) add_into(tot, grp);
+          if (G == 1) end_of_group();
         }
       }
     }
     if (it + 1 < n_tiles) put((it + 1) & 1);
     __syncthreads();
   }
-  add_into(grp, acc);  // what is left of the last slice (zeros after a whole one)
-  add_into(tot, grp);
+  end_of_slice();  // what is left of the last slice (zeros after a whole one)
   if constexpr (G > 1) {  // the sets' sums meet in shared memory, in order
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < TM; ++i)
       *reinterpret_cast<float4*>(smem + (set * BM + tm + i) * BN + tn) =
-          make_float4(tot[i][0], tot[i][1], tot[i][2], tot[i][3]);
+          make_float4(grp[i][0], grp[i][1], grp[i][2], grp[i][3]);
     __syncthreads();
     for (int o = threadIdx.x; o < BM * BN; o += G * SET) {
       const int m = m0 + o / BN, n = n0 + o % BN;
@@ -261,14 +279,17 @@ __global__ void __launch_bounds__(G * (BM / 4) * (BN / 4)) tiles_kernel(const Ar
       if (m < p.T && n < p.N) p.out[(size_t)m * p.N + n] = total + (p.bias ? p.bias[n] : 0.f);
     }
   } else {
+    end_of_group();
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < TM; ++i) {
       const int m = m0 + tm + i;
       if (m >= p.T) continue;
+      const float4 t = mine[i * SET];
+      const float v[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int n = n0 + tn + j;
-        if (n < p.N) p.out[(size_t)m * p.N + n] = tot[i][j] + (p.bias ? p.bias[n] : 0.f);
+        if (n < p.N) p.out[(size_t)m * p.N + n] = v[j] + (p.bias ? p.bias[n] : 0.f);
       }
     }
   }
@@ -285,11 +306,15 @@ static cudaError_t launch_few(const Args& p, cudaStream_t stream) {
   return lse::launch(few_rows_kernel<NPT, NG>, grid, 32 * NG, smem, stream, p);
 }
 
-template <int BM, int BN, int G>
+template <int BM, int BN, int TM, int G, int BLOCKS>
 static cudaError_t launch_tiles(const Args& p, bool vec, cudaStream_t stream) {
+  constexpr int smem = (G * 2 * BK * (BM + BN + 8) + (G == 1 ? BM * BN : 0)) * 4;
+  static const cudaError_t configured =
+      cudaFuncSetAttribute(tiles_kernel<BM, BN, TM, G, BLOCKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (configured != cudaSuccess) return configured;
   const dim3 grid((p.N + BN - 1) / BN, (p.T + BM - 1) / BM);
   if (grid.y > 65535) return cudaErrorInvalidValue;
-  return lse::launch(tiles_kernel<BM, BN, G>, grid, G * (BM / 4) * (BN / 4), 0, stream, p, vec);
+  return lse::launch(tiles_kernel<BM, BN, TM, G, BLOCKS>, grid, G * (BM / TM) * (BN / 4), smem, stream, p, vec);
 }
 
 }  // namespace gf32
@@ -302,16 +327,30 @@ extern "C" int lse_gemm_f32(const float* a, const float* w, const float* bias, f
   if (K <= 0 || (T + 63) / 64 > 65535) return LSE_BAD_ARGUMENT;
   const Args p{a, w, bias, out, T, N, K, slice_len(K), w_early};
   const bool vec = K % 4 == 0 && ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
-  // Measured alone with w out of L2, few rows / tiles in us (each with 6 us of start and timing), N x K, before /
-  // with more rows: 960 x 576 10 / 18 at 16 rows, 16 / 18 at 64; 3072 x 576 16 / 20 at 16, 33 / 27 at 64;
-  // 2048 x 2048 22 / 41 at 16, 35 / 41 at 32, 49 / 41 at 48; 16384 x 2048 72 / 96 at 8, 115 / 98 at 16, 166 / 100 at
-  // 24; 49152 x 576 64 / 137 at 8, 111 / 137 at 16, 174 / 137 at 24. A pass of 8 rows costs as much as the first
-  // one where w is large, almost nothing where the blocks are too few to fill the SMs.
-  const bool few = vec && (T <= 16 || (T <= 32 && N <= 4096));
-  // 64 x 64 tiles once they give every SM two blocks (900 rows, 3072 x 576: 125 us, 26 TFLOP/s); below that 32 x 32
-  const bool wide = (long long)((T + 63) / 64) * ((N + 63) / 64) >= 2 * 148 || (T + 31) / 32 > 65535;
-  const cudaError_t e = few    ? launch_few<4, 4>(p, stream)
-                        : wide ? launch_tiles<64, 64, 1>(p, vec, stream)
-                               : launch_tiles<32, 32, 4>(p, vec, stream);
+  // Blocks come to the SMs in rounds of 148, and a product takes about (a start) + (rounds) x (a block's share of an SM).
+  // With the constants below (tenths of a us at K = 576; all grow with K alike, the small tiles a little less) the
+  // choice was within 2.7 % of the best of the four in the mean of 316 products (N 576 to 49152, K 576 to 8192, 1 to
+  // 2048 rows) and nowhere slower than a kernel of 64 x 64 tiles with one chain of additions, but for 4 % of a K that
+  // is no multiple of 4. Alone with w out of L2, few rows / small / 64 x 64 / 64 x 128, us:
+  //   16384 x 576   8 rows 29 / 41 / 49 / 49    32 rows 74 / 43 / 49 / 49    128 rows - / 127 / 96 / 80
+  //   2048 x 2048   16 rows 22 / 41 / 104 / 139    300 rows - / 128 / 152 / 150    900 rows - / 307 / 307 / 250
+  //   3072 x 576    24 rows 18 / 20 / 35 / 47    900 rows - / 164 / 113 / 121    2048 rows - / 363 / 238 / 221
+  //   49152 x 576   8 rows 64 / 100 / 127 / 117    48 rows - / 186 / 131 / 119    900 rows - / 2578 / 1613 / 1388
+  auto rounds = [&](int bm, int bn) {
+    const long long blocks = (long long)((T + bm - 1) / bm) * ((N + bn - 1) / bn);
+    return (blocks + 147) / 148;
+  };
+  const long long small = 100 + (K >= 1024 ? 70 : 80) * rounds(32, 32);
+  const long long square = 180 + 200 * rounds(64, 64), wide = 100 + 360 * rounds(64, 128);
+  const long long few = vec && T <= 32 ? 80 + 22 * rounds(FEW_T, 16) : LLONG_MAX;
+  const long long tiles = square < wide ? square : wide;
+  // small tiles: where no SM gets more than two blocks they may have the registers of four (123 instead of 64 a thread:
+  // 6 to 11 % faster there, 6 % slower with more blocks)
+  const bool airy = rounds(32, 32) <= 2;
+  const cudaError_t e = few <= small && few <= tiles               ? launch_few<4, 4>(p, stream)
+                        : small <= tiles && (T + 31) / 32 <= 65535 ? (airy ? launch_tiles<32, 32, 4, 4, 2>(p, vec, stream)
+                                                                           : launch_tiles<32, 32, 4, 4, 4>(p, vec, stream))
+                        : square <= wide                           ? launch_tiles<64, 64, 4, 1, 3>(p, vec, stream)
+                                                                   : launch_tiles<64, 128, 8, 1, 2>(p, vec, stream);
   return e == cudaSuccess ? LSE_OK : LSE_LAUNCH_FAILED;
 }

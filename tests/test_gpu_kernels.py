@@ -100,6 +100,22 @@ def test_gemm_f32_every_kernel_adds_in_the_same_order(ops, N, K):
         assert torch.equal(run(a[first : first + n]), whole[first : first + n]), (first, n)
 
 
+@pytest.mark.parametrize("N,K", [(4850, 576), (4850, 1536), (4850, 1001),      # 320 rows: tiles of 64 x 64
+                                 (16400, 576), (9500, 1001), (9500, 1044),     # 64 x 128
+                                 (2000, 2308)])                               # 32 x 32
+def test_gemm_f32_long_slices_in_every_kernel(ops, N, K):
+    """As the test above with slices longer than eight (they end inside a tile of K) and more than two groups."""
+    w, b, a = rnd(N, K, seed=2).cuda(), rnd(N, seed=3).cuda(), rnd(320, K, seed=1).cuda()
+    run = lambda rows: ops.linear(rows.clone(), w, b, out_dtype=torch.float32)
+    whole = run(a)
+    ref = a.double() @ w.double().T + b.double()
+    size = a.double().abs() @ w.double().abs().T + b.double().abs()
+    chain = -(-K // 256) * 8 + 8 + 4 + 1
+    assert ((whole.double() - ref).abs() <= 1.01 * chain * 2.0**-24 * size).all()
+    for first, n in ((0, 1), (3, 8), (7, 16), (100, 32), (200, 33), (255, 65), (120, 200)):
+        assert torch.equal(run(a[first : first + n]), whole[first : first + n]), (first, n)
+
+
 @pytest.mark.parametrize("T", [1, 9, 40])
 def test_gemm_f32_with_weights_of_the_kernel_before(ops, T):
     """Both operands may be what a kernel of this package, launched just before, still writes; a parameter, which is
