@@ -975,7 +975,7 @@ void decay_linear_attention(const Tensor& proj, Tensor& out, Tensor& state, cons
                             const Tensor& ctx_lens, const Tensor& slots, int64_t H, int64_t dk, int64_t dv,
                             const OptTensor& cos, const OptTensor& sin, bool silu, double key_scale,
                             int64_t max_chunks, const OptTensor& chunks, const OptTensor& gate_z,
-                            double decay_root, double query_scale) {
+                            double decay_root, double query_scale, bool products) {
   check_f32(proj, "proj");
   check_f32(out, "out");
   check_state(state, "state", dk);
@@ -1025,7 +1025,7 @@ void decay_linear_attention(const Tensor& proj, Tensor& out, Tensor& state, cons
                                   cos ? cos->data_ptr<float>() : nullptr, sin ? sin->data_ptr<float>() : nullptr, rot,
                                   silu ? 1 : 0, (float)key_scale, (int)max_chunks, chunk_ptr, stream(),
                                   gate_z ? gate_z->data_ptr<float>() : nullptr, gate_z ? gate_z->size(1) : 0,
-                                  (float)decay_root, (float)query_scale, chunk_decay, (int)proj.size(0)),
+                                  (float)decay_root, (float)query_scale, chunk_decay, (int)proj.size(0), products ? 1 : 0),
        "decay_linear_attention");
 }
 
@@ -1514,7 +1514,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("decay_linear_attention", &decay_linear_attention, py::arg("proj"), py::arg("out"), py::arg("state"),
         py::arg("decay"), py::arg("cu_q"), py::arg("ctx_lens"), py::arg("slots"), py::arg("H"), py::arg("dk"),
         py::arg("dv"), py::arg("cos"), py::arg("sin"), py::arg("silu"), py::arg("key_scale"), py::arg("max_chunks"),
-        py::arg("chunks"), py::arg("gate_z") = py::none(), py::arg("decay_root") = 1.0, py::arg("query_scale") = 1.0);
+        py::arg("chunks"), py::arg("gate_z") = py::none(), py::arg("decay_root") = 1.0, py::arg("query_scale") = 1.0,
+        py::arg("products") = true);
   m.def("streams_spread", &streams_spread);
   m.def("streams_read_norm", &streams_read_norm);
   m.def("streams_write", &streams_write);

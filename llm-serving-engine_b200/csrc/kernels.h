@@ -201,7 +201,9 @@ int lse_decay_linear_attention(const float* proj, long long stride, float* out, 
                                // total_rows: rows of proj and gate_z. With max_chunks > 1 and total_rows > 0
                                // gate_z is overwritten with the decays (it is the caller's temporary).
                                const float* gate_z = nullptr, long long gate_stride = 0, float decay_root = 1.f,
-                               float query_scale = 1.f, float* chunk_decay = nullptr, int total_rows = 0);
+                               float query_scale = 1.f, float* chunk_decay = nullptr, int total_rows = 0,
+                               // 1: chunks as matrix products where the sizes allow it (linear_chunks.cuh)
+                               int products = 1);
 // ---- the gated delta rule (delta_rule.cu)
 
 // What enters the recurrence, from rows of proj (row length `stride`): q (G*dk) | k (G*dk) | v (H*dv) |

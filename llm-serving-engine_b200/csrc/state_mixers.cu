@@ -1038,7 +1038,7 @@ extern "C" int lse_decay_linear_attention(const float* proj, long long stride, f
                                           float key_scale, int max_chunks, float* chunks,
                                           cudaStream_t stream, const float* gate_z, long long gate_stride,
                                           float decay_root, float query_scale, float* chunk_decay,
-                                          int total_rows) {
+                                          int total_rows, int products) {
   if (num_seqs <= 0) return LSE_OK;
   if ((!gate_z && !decay) || (gate_z && (decay_root <= 0.f || gate_stride < (long long)H * dk)) ||
       (gate_z && max_chunks > 1 && !chunk_decay))
@@ -1078,7 +1078,7 @@ extern "C" int lse_decay_linear_attention(const float* proj, long long stride, f
   a.L = lse_linear_attention_chunk();
   a.phase = 0;
   a.short_only = 0;
-  if (!gated && max_chunks > 1) {
+  if (!gated && max_chunks > 1 && products) {
     // a decay per head: the chunks of long portions as matrix products (linear_chunks.cuh), where the sizes allow it
     lac::Args m;
     m.proj = proj; m.stride = stride; m.out = out; m.state = state; m.chunks = chunks; m.decay = decay;

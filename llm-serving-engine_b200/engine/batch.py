@@ -68,6 +68,7 @@ class DeviceStep:
     plans: dict[Any, dict[str, Any]]
     host: HostStep | None = None
     max_portion_ctx: int = 0  # bound of the contexts of the sequences with more than one token (0: not known)
+    portion_slots: int = 0  # a captured step: how many sequences of more than one token it has room for, padding included
     every_row_wanted: bool = False  # logit_rows is 0, 1, ..., num_tokens - 1: the final norm need not gather
 
 

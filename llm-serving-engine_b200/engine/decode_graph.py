@@ -167,7 +167,7 @@ class _MixedGraph:
             first_portion=view("first_portion"),
             block_tables=[view(("table", gi)).view(N, -1) for gi in range(len(runner.manager.groups))],
             logit_rows=view("logit_rows"), num_tokens=T, num_seqs=N, num_logit_rows=N,
-            max_decode_ctx=0, decode_splits=splits, max_portion_ctx=max_portion_ctx,
+            max_decode_ctx=0, decode_splits=splits, max_portion_ctx=max_portion_ctx, portion_slots=slots,
             plans={key: {name: view(("plan", key, name)).view(a.shape) for name, a in plan.items()}
                    for key, plan in plans.items()},
             host=None,

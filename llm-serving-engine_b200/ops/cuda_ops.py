@@ -142,6 +142,7 @@ class CudaOps:
         self.num_sms = torch.cuda.get_device_properties(self.device).multi_processor_count
         # 0: fastest available; 1: CUDA cores; 2: mma.sync fed by plain loads; 3: single tokens fed by TMA
         self.attention_kernel = 0  # (tests compare them)
+        self.linear_attention_products: bool | None = None  # (tests compare them; None: the faster one)
         self.use_skinny_gemm = True
         # rows up to which the own tcgen05 product runs (measured: above it the library is faster)
         self.skinny_max_rows = int(self.ext.gemm_bf16_skinny_max_rows())
@@ -797,10 +798,34 @@ class CudaOps:
             kept.append(torch.empty(need, dtype=torch.float32, device=self.device))
         return kept[-1]
 
+    @staticmethod
+    def _chunk_products(step, T: int, L: int, num_heads: int, large: bool) -> bool:
+        """Run the chunks of portions of more than ``L`` tokens as matrix products, or as the recurrence side by side?
+        The products take the time of a whole chunk however few tokens the last one has, and the sequences of at most
+        ``L`` tokens come in a launch after theirs, where the recurrence takes both in one. us, recurrence / products:
+        16 heads of 128 x 128, 65 tokens 41 / 60, 96 tokens 54 / 60, 128 tokens 69 / 58, four of 65 tokens 84 / 69, 16 of
+        65 tokens 245 / 149, 8 of 60 tokens beside one of 80 82 / 103, beside one of 300 155 / 124; 4 heads of 128 x 128,
+        four of 65 tokens 42 / 62, 16 of 65 tokens 87 / 70; 8 heads of 64 x 64, 65 tokens 26 / 25, 8 of 32 tokens beside
+        one of 80 33 / 41, beside one of 300 63 / 53. (``large``: a key or value size beyond 64.)"""
+        host = getattr(step, "host", None)
+        if host is not None:
+            lens = host.q_lens.tolist()
+            longest, short = max(lens), max((n for n in lens if n <= L), default=0)
+            chunks = sum(-(-n // L) for n in lens if n > L)
+        else:  # a captured step: portion slots of which one is for padding, filled about evenly
+            n = int(step.cu_q.shape[0]) - 1
+            slots = getattr(step, "portion_slots", 0)
+            longest, short = ((T - (n - slots)) // max(1, slots - 1), 2) if slots else (T - (n - 1), 0)
+            chunks = (T - n) // L
+        busy = large and num_heads * chunks >= 128
+        if short:
+            return busy or longest >= 80 + 3 * short
+        return busy or not large or longest >= 104
+
     def decay_linear_attention(self, proj, *, num_heads, key_dim, value_dim, decay, state, step,
                                activation, key_scale, cos, sin, decay_logits=None, decay_root=1.0,
                                query_scale=1.0):
-        """Portions longer than the kernel's chunk run as chunks side by side (three launches and
+        """Portions longer than the kernel's chunk run as chunks side by side (in several launches, with
         a scratch for the chunks' states); steps of single tokens and short portions are one launch.
         With ``decay_logits`` (float32 ``[T, heads * key_dim]``; ``decay`` is then None) the decay of
         key channel i at token t is ``sigmoid(z)^(1 / decay_root)``. ``query_scale`` multiplies q."""
@@ -816,11 +841,18 @@ class CudaOps:
             per_chunk = num_heads * (value_dim * key_dim + (key_dim if decay_logits is not None else 0))
             need = (T // L + int(step.cu_q.shape[0]) - 1) * per_chunk
             scratch = self._kept_scratch("linear attention", need)
+        sizes_fit = (max(key_dim, value_dim) <= 128 and key_dim % 4 == 0 and value_dim % 4 == 0 and proj.shape[1] % 4 == 0)
+        products = max_chunks > 1 and decay_logits is None and sizes_fit and (
+            self._chunk_products(step, T, L, num_heads, max(key_dim, value_dim) > 64)
+            if self.linear_attention_products is None else self.linear_attention_products)
         self.ext.decay_linear_attention(proj, out, state, decay, step.cu_q, step.ctx_lens, step.state_slots,
                                         num_heads, key_dim, value_dim, cos, sin, activation == "silu",
                                         float(key_scale), max_chunks, scratch, decay_logits, float(decay_root),
-                                        float(query_scale))
-        self.launches += 3 if max_chunks > 1 else 1
+                                        float(query_scale), products)
+        if decay_logits is not None:
+            self.launches += 5 if max_chunks > 1 else 1
+        else:  # with products the sequences of at most a chunk have a launch of their own
+            self.launches += (1 if max_chunks == 1 else 3 if not products or step.cu_q.shape[0] == 2 else 4)
         return out
 
     # ------------------------------------------------------------------ gated delta rule

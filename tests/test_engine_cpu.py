@@ -390,6 +390,27 @@ def test_float32_context_partitions_change_once_per_doubling(group, blocks_per_s
             last = top + 1
 
 
+@pytest.mark.parametrize("lens,heads,large,products", [
+    ([65], 16, True, False), ([104], 16, True, True), ([65] * 4, 16, True, True), ([65] * 4, 4, True, False),
+    ([65], 8, False, True), ([60] * 8 + [200], 8, False, False), ([60] * 8 + [260], 8, False, True),
+    ([60] * 8 + [80], 16, True, False), ([1] * 8 + [100], 8, False, True), ([2000], 16, True, True)])
+def test_how_chunks_of_linear_attention_run(lens, heads, large, products):
+    """Each line of the rule from both sides; the captured step of the same portions, one by one, decides alike."""
+    from types import SimpleNamespace
+
+    import numpy as np
+    import torch
+
+    from llmserve_b200.ops.cuda_ops import CudaOps
+
+    step = SimpleNamespace(host=SimpleNamespace(q_lens=np.array(lens)), cu_q=torch.zeros(len(lens) + 1))
+    assert CudaOps._chunk_products(step, sum(lens), 64, heads, large) is products
+    for n in (70, 200, 900):
+        alone = SimpleNamespace(host=SimpleNamespace(q_lens=np.array([1, 1, n, 2])), cu_q=torch.zeros(5))
+        captured = SimpleNamespace(host=None, cu_q=torch.zeros(5), portion_slots=2)
+        assert CudaOps._chunk_products(captured, n + 4, 64, 16, True) is CudaOps._chunk_products(alone, n + 4, 64, 16, True)
+
+
 def test_context_partitions_fill_whole_waves():
     """148 SMs holding 7 blocks each run 1036 blocks at a time. The number of partitions per
     (sequence, head) avoids a last wave that is nearly empty, keeps partitions of 128 keys or

@@ -172,6 +172,26 @@ def test_linear_attention_chunk_products_at_their_edges(ops, H, dk, dv, rot, sil
     assert bool((state[[4, 6]] == 1e4).all())
 
 
+@pytest.mark.parametrize("products", [False, True])
+@pytest.mark.parametrize("lens", [[65], [128, 129], [60, 80, 1], [64, 200, 33]])
+def test_linear_attention_either_way_of_running_chunks(ops, monkeypatch, lens, products):
+    """The recurrence and the matrix products over chunks serve the same steps: short sequences beside long ones,
+    continued from a state, activated (rows beyond a portion's end are not)."""
+    H, dk, dv, decay = 3, 32, 64, [0.999, 0.9, 0.5]
+    monkeypatch.setattr(ops, "linear_attention_products", products)
+    kw = dict(num_heads=H, key_dim=dk, value_dim=dv, decay=torch.tensor(decay).cuda(), activation="silu",
+              key_scale=dk ** -0.5, cos=None, sin=None)
+    seqs = [rnd(5 + n, 2 * H * dk + H * dv, seed=60 + i, scale=0.7) for i, n in enumerate(lens)]
+    state, slots, k = torch.full((4, H, dv, dk), 1e4).cuda(), list(range(len(lens))), len(lens)
+    before = ops.launches
+    ops.decay_linear_attention(torch.cat([s[:5] for s in seqs]).cuda(), state=state, step=batch([5] * k, [0] * k, slots), **kw)
+    assert ops.launches - before == 1
+    out = ops.decay_linear_attention(torch.cat([s[5:] for s in seqs]).cuda(), state=state, step=batch(lens, [5] * k, slots), **kw)
+    assert ops.launches - before == 1 + (3 if not products or k == 1 else 4)
+    for s, o in zip(seqs, out.split(lens)):
+        close(o, linear_attention_reference(s, H, dk, dv, decay, True, 0, 0, dk ** -0.5)[5:], 2e-5)
+
+
 @pytest.mark.parametrize("bad", [float("nan"), float("inf")])
 @pytest.mark.parametrize("at", [1, 15, 16, 50, 63, 64, 100])
 def test_linear_attention_chunk_products_know_nothing_of_later_tokens(ops, at, bad):
