@@ -16,6 +16,8 @@
 // 149 us (sums 40, chain 41 from memory, outputs 106 with cold caches, overlapped).
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace lse {
@@ -375,8 +377,9 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_outputs_kernel(const Args a)
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int m = 0; m < M; ++m) part[i][m] = 0.f;
-#pragma unroll 1
-    for (int t = 16 * b; t < 16 * b + 16; t += 4) {
+    // A later token's value is left out of the row's own block and not only met by a zero: it may be no number. A warp
+    // has two rows of each block, so four tokens are all of them before, all of them behind, or looked at one by one.
+    auto four = [&](int t, auto own) {
       float p[4][4];
 #pragma unroll
       for (int i = b; i < 4; ++i) load4<float>(qs + (ty + 16 * i) * LDP + t, p[i]);
@@ -385,12 +388,19 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_outputs_kernel(const Args a)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const float v = vs[(t + e) * LDV + tx + 16 * m];
-          // a later token's value is left out and not only met by a zero: it may be no number
-          part[b][m] = fmaf(p[b][e], t + e <= ty + 16 * b ? v : 0.f, part[b][m]);
+          if constexpr (own.value == 2) part[b][m] = fmaf(p[b][e], v, part[b][m]);
+          if constexpr (own.value == 1) part[b][m] = fmaf(p[b][e], t + e <= ty + 16 * b ? v : 0.f, part[b][m]);
 #pragma unroll
           for (int i = b + 1; i < 4; ++i) part[i][m] = fmaf(p[i][e], v, part[i][m]);
         }
-    }
+    };
+    const int mixed = 16 * b + (ty & ~3);  // (the same for both rows of the warp)
+#pragma unroll 1
+    for (int t = 16 * b; t < mixed; t += 4) four(t, std::integral_constant<int, 2>());
+    four(mixed, std::integral_constant<int, 1>());
+    if (b < 3)
+#pragma unroll 1
+      for (int t = mixed + 4; t < 16 * b + 16; t += 4) four(t, std::integral_constant<int, 0>());
 #pragma unroll
     for (int i = b; i < 4; ++i)
 #pragma unroll
