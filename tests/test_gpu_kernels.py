@@ -423,6 +423,61 @@ def test_prefill_attention_shared_by_clusters(ops, nq, nk, q_lens, ctx_lens, pag
     ops.check_kernel_errors()
 
 
+@pytest.mark.parametrize("options", ["plain", "sinks", "cap", "window 600", "chunk 600", "window 650 sinks cap", "chunk 700 sinks"])
+@pytest.mark.parametrize("nq,nk,q_lens,ctx_lens,page", [
+    (2, 1, [130], [901], 16),                    # 4 blocks: four share a tile's keys
+    (24, 8, [128, 129], [790, 1100], 64),        # 72: two do
+    (40, 8, [200, 300], [700, 900], 8)])         # 200: nothing is shared
+def test_prefill_attention_options_shared_by_clusters(ops, options, nq, nk, q_lens, ctx_lens, page):
+    """Sinks, soft caps, windows and chunks under every way of sharing the keys. Whatever lies beside the keys that some
+    row sees (after the context, before a window or a chunk, on pages no longer held) is not a number. Bound: the
+    probabilities and the result are each rounded once to bfloat16 (8 bits: at most 2^-8 of the value), the rest is float32."""
+    words = options.split()
+    value = lambda name: int(words[words.index(name) + 1]) if name in words else 0
+    window, chunk, cap = value("window"), value("chunk"), 8.0 if "cap" in words else 0.0
+    g = torch.Generator().manual_seed(nq + len(options))
+    sinks = 6 + 2 * torch.randn(nq, generator=g) if "sinks" in words else None
+    D, n = 64, len(q_lens)
+    first = lambda p: max(p - window + 1 if window else 0, p // chunk * chunk if chunk else 0, 0)
+    pages = [-(-c // page) for c in ctx_lens]
+    kp, vp = (torch.full((sum(pages) + 1, nk, page, D), float("nan"), dtype=torch.bfloat16) for _ in range(2))
+    order = torch.randperm(sum(pages) + 1, generator=g)
+    tables = torch.full((n, max(pages)), int(order[-1]), dtype=torch.int32)  # (a page that nobody holds)
+    q = (1.5 * torch.randn(sum(q_lens), nq * D, generator=g)).bfloat16()
+    want, bound, at, used = [], [], 0, 0
+    for s, (ql, c) in enumerate(zip(q_lens, ctx_lens)):
+        lo = first(c - ql)
+        for b in range(lo // page, pages[s]):
+            tables[s, b] = order[used + b]
+        used += pages[s]
+        k, v = (torch.randn(c, nk, D, generator=g).bfloat16() for _ in range(2))
+        for p in range(lo, c):
+            kp[tables[s, p // page], :, p % page], vp[tables[s, p // page], :, p % page] = k[p], v[p]
+        j = torch.arange(c)
+        hidden = torch.stack([(j > p) | (j < first(p)) for p in range(c - ql, c)])
+        k, v = (x.double().repeat_interleave(nq // nk, 1).transpose(0, 1) for x in (k, v))
+        sc = q[at : at + ql].double().view(ql, nq, D).transpose(0, 1) @ k.transpose(1, 2) * 0.125
+        sc = (cap * torch.tanh(sc / cap) if cap else sc).masked_fill(hidden, float("-inf"))
+        if sinks is not None:
+            sc = torch.cat([sc, sinks.double()[:, None, None].expand(nq, ql, 1)], 2)
+        w = sc.softmax(-1)[:, :, :c]
+        rows = lambda x: x.transpose(0, 1).reshape(ql, nq * D)
+        want.append(rows(w @ v))
+        bound.append(rows(w @ v.abs()) + want[-1].abs())
+        at += ql
+    cu = np.concatenate([[0], np.cumsum(q_lens)]).astype(np.int32)
+    step = SimpleNamespace(cu_q=torch.from_numpy(cu).cuda(), ctx_lens=torch.tensor(ctx_lens, dtype=torch.int32),
+                           q_lens=np.asarray(q_lens, dtype=np.int32), decode_splits=0, max_decode_ctx=0)
+    ops.check_attention_shape(D, torch.bfloat16)
+    plan = {k: torch.from_numpy(v).cuda() for k, v in ops.attention_plan(step, torch.bfloat16, D).items()}
+    step.ctx_lens = step.ctx_lens.cuda()
+    got = ops.paged_attention(q.cuda(), num_heads=nq, num_kv_heads=nk, head_dim=D, scale=0.125, window=window, chunk=chunk,
+                              sinks=None if sinks is None else sinks.cuda(), softcap=cap, k_pages=kp.cuda(), v_pages=vp.cuda(),
+                              block_tables=tables.cuda(), page_tokens=page, step=step, plan=plan).double().cpu()
+    ops.check_kernel_errors()
+    assert ((got - torch.cat(want)).abs() <= 1.01 * 2.0**-8 * torch.cat(bound) + 1e-5).all()
+
+
 @pytest.mark.parametrize("nq,nk,q_lens,ctx_lens", [(2, 1, [100], [300]), (24, 8, [129, 2, 128], [500, 2, 449])])
 def test_prefill_attention_of_short_contexts_under_wide_tables(ops, nq, nk, q_lens, ctx_lens):
     """Block tables as wide as the longest request allowed, as captured steps have them: with the contexts' bound known
