@@ -581,9 +581,7 @@ template <bool CAP, int PARTS, bool LOCAL>
 inline int launch_prefill_parts(const LseAttnArgs* a, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
                                 const Params& p, cudaStream_t stream) {
   constexpr int smem = Q_BYTES + 2 * STAGES * KV_BYTES + (2 * STAGES + 6) * 8 + 16 + 1024;
-  static const cudaError_t configured =
-      cudaFuncSetAttribute(prefill_tc_kernel<CAP, PARTS, LOCAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (configured != cudaSuccess) return LSE_LAUNCH_FAILED;
+  if (lse::allow_dynamic_smem<prefill_tc_kernel<CAP, PARTS, LOCAL>, smem>() != cudaSuccess) return LSE_LAUNCH_FAILED;
   const dim3 grid(a->num_heads * PARTS, a->num_tiles);
   return lse::launch_clusters(prefill_tc_kernel<CAP, PARTS, LOCAL>, grid, THREADS, PARTS, smem, stream, mq, mk, mv, p) == cudaSuccess
              ? LSE_OK

@@ -6,6 +6,8 @@
 #include <stdint.h>
 #include <stdlib.h>
 
+#include <atomic>
+
 #include "status.h"
 
 namespace lse {
@@ -174,6 +176,20 @@ inline cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+
+// Lets KERNEL have up to BYTES of dynamic shared memory. The attribute is a device's, so it is set once on each.
+template <auto KERNEL, int BYTES>
+inline cudaError_t allow_dynamic_smem() {
+  static std::atomic<unsigned long long> set{0};
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  const unsigned long long bit = device < 64 ? 1ull << device : 0;
+  if (set.load(std::memory_order_relaxed) & bit) return cudaSuccess;
+  e = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, BYTES);
+  if (e == cudaSuccess) set.fetch_or(bit, std::memory_order_relaxed);
+  return e;
 }
 
 // The same in clusters of `cluster` blocks along x.

@@ -299,9 +299,7 @@ template <int NPT, int NG>
 static cudaError_t launch_few(const Args& p, cudaStream_t stream) {
   constexpr int NB = NPT * NG, smem = STAGES * (NB + FEW_T) * ROW * 4;
   static_assert(FEW_T * NB * (SLICES + 1) * 4 <= smem, "");
-  static const cudaError_t configured =
-      cudaFuncSetAttribute(few_rows_kernel<NPT, NG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (configured != cudaSuccess) return configured;
+  if (const cudaError_t e = allow_dynamic_smem<few_rows_kernel<NPT, NG>, smem>()) return e;
   const dim3 grid((p.N + NB - 1) / NB, (p.T + FEW_T - 1) / FEW_T);
   return lse::launch(few_rows_kernel<NPT, NG>, grid, 32 * NG, smem, stream, p);
 }
@@ -309,9 +307,7 @@ static cudaError_t launch_few(const Args& p, cudaStream_t stream) {
 template <int BM, int BN, int TM, int G, int BLOCKS>
 static cudaError_t launch_tiles(const Args& p, bool vec, cudaStream_t stream) {
   constexpr int smem = (G * 2 * BK * (BM + BN + 8) + (G == 1 ? BM * BN : 0)) * 4;
-  static const cudaError_t configured =
-      cudaFuncSetAttribute(tiles_kernel<BM, BN, TM, G, BLOCKS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (configured != cudaSuccess) return configured;
+  if (const cudaError_t e = allow_dynamic_smem<tiles_kernel<BM, BN, TM, G, BLOCKS>, smem>()) return e;
   const dim3 grid((p.N + BN - 1) / BN, (p.T + BM - 1) / BM);
   if (grid.y > 65535) return cudaErrorInvalidValue;
   return lse::launch(tiles_kernel<BM, BN, TM, G, BLOCKS>, grid, G * (BM / TM) * (BN / 4), smem, stream, p, vec);

@@ -424,16 +424,10 @@ inline bool serves(const Args& a) {
          aligned(a.state) && aligned(a.chunks) && aligned(a.cos) && aligned(a.sin) && a.H <= 65535;
 }
 
-template <auto KERNEL, int MOST>
-inline bool allow() {
-  static const bool ok = cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST) == cudaSuccess;
-  return ok;
-}
-
 template <int VH, int KH>
 inline bool launch_sums(const Args& a, dim3 grid, cudaStream_t stream) {
   constexpr int smem = L * 64 * (VH + KH) * 4;
-  return allow<chunk_sums_kernel<VH, KH>, smem>() &&
+  return allow_dynamic_smem<chunk_sums_kernel<VH, KH>, smem>() == cudaSuccess &&
          launch(chunk_sums_kernel<VH, KH>, grid, THREADS, smem, stream, a) == cudaSuccess;
 }
 template <int M>
@@ -441,7 +435,7 @@ inline bool launch_outputs(const Args& a, dim3 grid, cudaStream_t stream) {
   const int ld = a.dk + 4, first = 16 * M * ld, second = L * (ld + 16 * M);
   const int smem = (L * (a.dk > L ? ld : L + 4) + (first > second ? first : second)) * 4;
   constexpr int most = (L * (MAX + 4) + (16 * M > L ? 16 * M * (MAX + 4) : 0) + L * (MAX + 4 + 16 * M)) * 4;
-  return allow<chunk_outputs_kernel<M>, most>() &&
+  return allow_dynamic_smem<chunk_outputs_kernel<M>, most>() == cudaSuccess &&
          launch(chunk_outputs_kernel<M>, grid, THREADS, smem, stream, a) == cudaSuccess;
 }
 
