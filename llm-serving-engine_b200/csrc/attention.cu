@@ -16,8 +16,8 @@
 //
 // Kernels:
 //   prefill_simt  portions of >= 2 rows, any dtype: 32 rows per block, 4 threads per row.
-//   prefill_tc    (attention_tc.cuh) bfloat16 portions, D = 64, no window: tcgen05 tensor cores with
-//                 TMA-fed operands and accumulators in tensor memory.
+//   prefill_tc    (attention_tc.cuh) bfloat16 portions, D = 64, also with a window, chunks, sinks or a soft cap: tcgen05
+//                 tensor cores with TMA-fed operands and accumulators in tensor memory.
 //   prefill_mma   bfloat16 portions, D <= 128: 128 rows per block (8 warps) on mma.sync tensor
 //                 cores; key/value tiles of 64 tokens are double-buffered with cp.async.
 //   decode_split  single rows: the context is cut into partitions, one block per (partition,

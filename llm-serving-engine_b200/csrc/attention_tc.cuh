@@ -17,15 +17,18 @@
 //                    of a row writes half of the head dims.
 // A stream's reference maximum moves only when a row of the warp outgrows it by 2^8; only then is
 // its O rescaled in tensor memory (tcgen05.ld / st) before its next P V. Warps 0-3 are stream 0 and warps 4-7
-// stream 1 (warp w owns tensor-memory lanes 32 (w mod 4) ..), one lane of warp 8 runs the TMA
-// pipeline, one lane of warp 9 issues the MMAs. Every barrier wait is bounded.
+// stream 1 (warp w owns tensor-memory lanes 32 (w mod 4) ..), warp 8 looks the pages up and its lanes issue the
+// TMA copies, one lane of warp 9 issues the MMAs. Every mbarrier wait is bounded; the barriers of a cluster
+// are reached by every warp of every block behind its bounded waits.
 //
 // What bounds it: the exp unit (16 per clock and SM) and, short of that, the latencies of a tile: wait, tcgen05.ld,
 // maximum, exponentials, tcgen05.st, arrival, P V, next Q K^T. A thread therefore takes 64 scores per round, the
 // two streams of a block are never in step, and two blocks share an SM. Pages of 16 tokens make eight copies per
 // tile; issued by one lane they were what a tile waited for. 2040 rows behind 6144 keys, 9 heads: 123 us (one lane
 // issuing, both streams on halves of one tile) -> 94 us -> 60 us with the keys shared by two blocks (exp unit alone:
-// 29 us); 2048 rows behind 4096 keys, 32 heads: 166 -> 141 us (75 us); 2048 rows alone, 32 heads: 45 -> 47 us (15 us).
+// 29 us); 2048 rows behind 4096 keys, 32 heads: 166 -> 141 us (75 us); 2048 rows alone, 32 heads: 45 -> 47 us by itself,
+// 37.6 -> 35.3 back to back (15 us). Short portions that just overflow the SMs lose: four of 700 rows, 15 heads (360
+// blocks) 16.5 -> 18.4, eight of 300 rows, 32 heads 22.9 -> 23.3.
 // 2048 rows, 32 heads, a window of 1024 with sinks: 41 us, chunks of 512: 29 us (mma.sync kernel: 125, 59).
 #pragma once
 
@@ -271,8 +274,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_consta
       int row_l = 0;
       if (t_l < n_tiles) {
         const int j = (t_first + t_l) * KT + b_l * p.box_rows;
-        // a box past the context re-reads the last valid page: its keys are masked anyway,
-        // and what it brings is finite
+        // a box past the context re-reads the last valid page, one before the first key the first page that is
+        // held: their keys are masked, and their values cleared before the multiply
         const int pi = max(min(j >> p.page_shift, last_page_idx), first_page_idx);
         const int off = (j >> p.page_shift) <= last_page_idx ? (j & (a.page_tokens - 1)) : 0;
         row_l = (table[pi] * a.num_kv_heads + kvh) * a.page_tokens + off;

@@ -12,7 +12,7 @@
 // token, had 2.1e-7 (16 heads of 128 x 128, 2048 tokens), and no faster (each split is four instructions).
 //
 // What bounds it: the 16-byte reads of shared memory in the outputs (four passes each, 48 for 128 multiply-adds of a
-// warp) and the FMA units; 2.7e9 multiply-adds at these sizes are 36 us at their peak. 269 us with the recurrence ->
+// warp) and the FMA units; 1.4e9 multiply-adds at these sizes are 36 us at their peak. 269 us with the recurrence ->
 // 149 us (sums 40, chain 41 from memory, outputs 106 with cold caches, overlapped).
 #pragma once
 
