@@ -2,10 +2,12 @@
 // contiguity of what it is given and raises on anything it cannot serve; work is enqueued on
 // PyTorch's current CUDA stream. Attention kernels live in one shared library per head size,
 // loaded here with dlopen.
+#include <ATen/TensorSubclassLikeUtils.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/tunable/Tunable.h>
 #include <cublas_v2.h>
 #include <dlfcn.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
 
 #include <algorithm>
@@ -241,8 +243,12 @@ void poly_norm(const Tensor& z, const Tensor& coef, double eps, Tensor& out) {
 // out = alpha a w^T (+ out) by the library, float32 sums, as torch.mm and torch.addmm call it by default: the same
 // function with the same arguments, without the views, the argument parsing and the dispatch in front of it. false:
 // torch's own call has to serve this one (nothing was done) -- empty or other than plain matrices, matrices of another
-// device than the current one, gradients, or any setting of torch's that changes which function it calls or how.
+// device than the current one, gradients (reverse or forward), tensors or modes through which torch follows its calls
+// (vmap, fake tensors, flop counts, traces), or any setting of torch's that changes which function it calls or how.
 bool gemm_bf16_library(const Tensor& a, const Tensor& w, Tensor& out, double alpha, bool accumulate) {
+  if (torch::jit::tracer::isTracing()) return false;
+  for (const Tensor* t : {&a, &w, static_cast<const Tensor*>(&out)})
+    if (at::isTensorSubclassLike(*t) || t->_fw_grad(0).defined()) return false;
   for (const Tensor* t : {&a, &w, static_cast<const Tensor*>(&out)})
     if (!t->is_cuda() || !t->is_contiguous() || t->dim() != 2 || t->device().index() != at::cuda::current_device()) return false;
   const int64_t T = a.size(0), N = w.size(0), K = a.size(1);

@@ -545,6 +545,25 @@ def test_library_product_follows_torchs_settings(ops, monkeypatch):
     assert ops.linear(a.requires_grad_(), w).requires_grad and len(calls) == 3
 
 
+def test_library_product_is_seen_by_whoever_follows_torchs_calls(ops):
+    """Forward derivatives, vmap, flop counts and traces of a product of many rows are those of torch.mm."""
+    import torch.autograd.forward_ad as forward
+    from torch.utils.flop_counter import FlopCounterMode
+
+    a, w, d = (rnd(n, 64, seed=i).bfloat16().cuda() for i, n in enumerate((40, 24, 40)))
+    with forward.dual_level():
+        got = forward.unpack_dual(ops.linear(forward.make_dual(a, d), w)).tangent
+    assert got is not None and torch.equal(got, torch.mm(d, w.t()))
+    with FlopCounterMode(display=False) as counted:
+        ops.linear(a, w)
+    assert counted.get_total_flops() == 2 * 40 * 24 * 64
+    # batches of matrices are another function of the library: each result is rounded once from float32
+    both, ref = torch.vmap(lambda x: ops.linear(x, w))(torch.stack([a, d])), torch.stack([a, d]).double() @ w.double().t()
+    assert ((both.double() - ref).abs() <= 2.0**-8 * ref.abs() + 64 * 2.0**-24 * (a.abs().max() * w.abs().max() * 64).item()).all()
+    traced = torch.jit.trace(lambda x: ops.linear(x, w), (a,), check_trace=False)
+    assert torch.equal(traced(d), torch.mm(d, w.t()))
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("window", [1, 5, 64, 100])
 def test_attention_window_edges(ops, dtype, window):
