@@ -1114,6 +1114,107 @@ void paged_attention_from_sums(Tensor& sums, Tensor& out, Tensor& k_pages, Tenso
   if (T > 0) done(lib.decode(&a, stream()), "paged_attention_from_sums");
 }
 
+// ------------------------------------------------------------------ a layer of few tokens
+bool few_tokens_serves(bool bf16, int64_t T, int64_t N, int64_t K, bool norm, bool pair) {
+  return std::max({T, N, K}) < (1 << 24) &&
+         lse_few_tokens_serves(bf16 ? LSE_BF16 : LSE_F32, (int)T, (int)N, (int)K, norm, pair) != 0;
+}
+
+// out = norm(x) @ w.T (norm_weight; pair: silu(gate) * up of it), or out = (x +) a @ w.T
+void few_tokens(const OptTensor& x, const OptTensor& norm_weight, double eps, const OptTensor& a, const Tensor& w, Tensor& out,
+                bool pair, bool w_early) {
+  check_cuda(w, "w");
+  check_cuda(out, "out");
+  const bool norm = norm_weight.has_value();
+  TORCH_CHECK(w.dim() == 2 && out.dim() == 2 && w.size(0) == out.size(1) * (pair ? 2 : 1),
+              "few_tokens: need w [N, K] (pair: [2 N, K]), out [T, N]");
+  const int64_t T = out.size(0), N = out.size(1), K = w.size(1);
+  const int code = dtype_code(w, "w");
+  TORCH_CHECK((code == LSE_F32 || code == LSE_BF16) && out.scalar_type() == (pair ? w.scalar_type() : torch::kFloat32),
+              "few_tokens: bad dtypes");
+  TORCH_CHECK(norm ? x.has_value() && !a : a.has_value() && !pair,
+              "few_tokens: a norm of x, perhaps for pairs, or a product of a");
+  if (x) {
+    check_f32(*x, "x");
+    TORCH_CHECK(x->dim() == 2 && x->size(0) == T && x->size(1) == (norm ? K : N) && x->data_ptr() != out.data_ptr(),
+                "few_tokens: x must be [T, K] of a norm or [T, N] beside a product, and not out");
+  }
+  if (norm) {
+    check_f32(*norm_weight, "norm_weight");
+    TORCH_CHECK(norm_weight->numel() == K, "few_tokens: norm_weight must be [K]");
+  } else {
+    check_cuda(*a, "a");
+    TORCH_CHECK(a->scalar_type() == w.scalar_type() && a->dim() == 2 && a->size(0) == T && a->size(1) == K,
+                "few_tokens: a must be [T, K] of w's dtype");
+  }
+  TORCH_CHECK(few_tokens_serves(code == LSE_BF16, T, N, K, norm, pair), "few_tokens: not served");
+  done(lse_few_tokens(x ? x->data_ptr<float>() : nullptr, norm ? norm_weight->data_ptr<float>() : nullptr, (float)eps,
+                      a ? a->data_ptr() : nullptr, w.data_ptr(), out.data_ptr(), code, (int)T, (int)N, (int)K, pair, w_early,
+                      stream()),
+       "few_tokens");
+}
+
+// Rotation, cache write and attention of single tokens from the rows of the projection; parts: room for the results of more
+// than one part of the context
+void few_attention(const Tensor& qkv, Tensor& out, const OptTensor& parts, Tensor& k_pages, Tensor& v_pages, int64_t num_heads, int64_t num_kv_heads,
+                   double scale, const Tensor& block_tables, const Tensor& ctx_lens, const Tensor& cu_q,
+                   const Tensor& decode_seqs, int64_t splits, const OptTensor& cos, const OptTensor& sin) {
+  constexpr int64_t D = 64;
+  check_f32(qkv, "qkv");
+  check_cuda(out, "out");
+  check_cuda(k_pages, "k_pages");
+  check_cuda(v_pages, "v_pages");
+  check_i32(block_tables, "block_tables");
+  check_i32(ctx_lens, "ctx_lens");
+  check_i32(cu_q, "cu_q");
+  check_i32(decode_seqs, "decode_seqs");
+  const int64_t T = qkv.size(0);
+  const int code = dtype_code(k_pages, "k_pages");
+  TORCH_CHECK(num_heads > 0 && num_kv_heads > 0 && qkv.dim() == 2 && qkv.size(1) == (num_heads + 2 * num_kv_heads) * D,
+              "few_attention: qkv must be [T, (heads + 2 kv_heads) * 64]");
+  TORCH_CHECK((code == LSE_F32 || code == LSE_BF16) && k_pages.dim() == 4 && k_pages.size(1) == num_kv_heads &&
+                  k_pages.size(3) == D && v_pages.sizes() == k_pages.sizes() && v_pages.scalar_type() == k_pages.scalar_type(),
+              "few_attention: pages must be [pages, kv_heads, page_tokens, 64]");
+  TORCH_CHECK(block_tables.dim() == 2 && cu_q.size(0) == ctx_lens.size(0) + 1 && block_tables.size(0) >= ctx_lens.size(0) &&
+                  decode_seqs.numel() == T,
+              "few_attention: per-sequence arrays disagree, or a row is not a single token");
+  TORCH_CHECK(cos.has_value() == sin.has_value(), "few_attention: cos and sin go together");
+  TORCH_CHECK(splits >= 1 && splits <= 4096 && T <= 64, "few_attention: bad number of parts");
+  TORCH_CHECK(out.scalar_type() == k_pages.scalar_type() && out.dim() == 2 && out.size(0) == T && out.size(1) == num_heads * D,
+              "few_attention: out must be [T, heads * 64] of the pages' dtype");
+  if (splits > 1) {
+    TORCH_CHECK(parts.has_value(), "few_attention: several parts need room for their results");
+    check_f32(*parts, "parts");
+    TORCH_CHECK(parts->numel() >= (int64_t)lse_few_attention_floats((int)T, (int)num_heads, (int)splits),
+                "few_attention: no room for the parts' results");
+  }
+  LseFewAttention a{};
+  a.dtype = code;
+  a.T = (int)T; a.H = (int)num_heads; a.KVH = (int)num_kv_heads;
+  a.page_tokens = (int)k_pages.size(2);
+  a.splits = (int)splits;
+  a.scale = (float)scale;
+  a.qkv = qkv.data_ptr<float>();
+  a.out = out.data_ptr();
+  if (splits > 1) a.parts = parts->data_ptr<float>();
+  a.k_pages = k_pages.data_ptr();
+  a.v_pages = v_pages.data_ptr();
+  if (cos) {
+    check_f32(*cos, "cos");
+    check_f32(*sin, "sin");
+    TORCH_CHECK(cos->dim() == 2 && cos->size(1) == D / 2 && sin->sizes() == cos->sizes(),
+                "few_attention: cos and sin must be [positions, 32]");
+    a.cos = cos->data_ptr<float>();
+    a.sin = sin->data_ptr<float>();
+  }
+  a.block_tables = block_tables.data_ptr<int>();
+  a.ctx_lens = ctx_lens.data_ptr<int>();
+  a.cu_q = cu_q.data_ptr<int>();
+  a.decode_seqs = decode_seqs.data_ptr<int>();
+  a.table_stride = (int)block_tables.size(1);
+  done(lse_few_attention(&a, stream()), "few_attention");
+}
+
 // ------------------------------------------------------------------ sampling
 void sample(const Tensor& logits, const Tensor& temperature, const Tensor& top_k,
             const Tensor& top_p, const Tensor& min_p, const Tensor& seed, const Tensor& draw,
@@ -1534,6 +1635,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("linear_attention_chunk", []() { return (int64_t)lse_linear_attention_chunk(); });
   m.def("paged_attention_from_sums", &paged_attention_from_sums);
   m.def("attention_takes_sums", &attention_takes_sums);
+  m.def("few_tokens", &few_tokens);
+  m.def("few_tokens_serves", &few_tokens_serves);
+  m.def("few_attention", &few_attention);
+  m.def("few_attention_floats", [](int64_t T, int64_t H, int64_t splits) { return (int64_t)lse_few_attention_floats((int)T, (int)H, (int)splits); });
   m.def("sample", &sample, py::arg("logits"), py::arg("temperature"), py::arg("top_k"), py::arg("top_p"),
         py::arg("min_p"), py::arg("seed"), py::arg("draw"), py::arg("out"), py::arg("scratch") = py::none(),
         py::arg("which") = 3);

@@ -89,6 +89,31 @@ int lse_gemm_bf16_skinny_max_rows(void);
 int lse_gemm_bf16_skinny(const void* a, const void* w, const void* bias, void* out, int T, int N,
                          int K, int* error_flag, cudaStream_t stream);
 
+// Products of at most sixteen tokens (float32: eight), with the norm before them or the residual add after them (few_tokens.cu):
+//   norm_weight [K] given: a = x / rms(x) * norm_weight rounded to `dtype` (the weights'), x float32 [T, K];
+//     out[T, N] = a . w[N, K]^T in float32, or with pair, w being [2 N, K] with gates above ups, silu(gate) * up in `dtype`;
+//   else out[T, N] = (x +) a[T, K] . w[N, K]^T in float32, a of `dtype`, x float32 [T, N] or null (out may not be x);
+// float32 products add in the order of lse_gemm_f32. w_early: as there.
+int lse_few_tokens_serves(int dtype, int T, int N, int K, int norm, int pair);
+int lse_few_tokens(const float* x, const float* norm_weight, float eps, const void* a, const void* w, void* out, int dtype,
+                   int T, int N, int K, int pair, int w_early, cudaStream_t stream);
+
+// Rotation, cache write and attention of T single tokens (head size 64, at most four query heads per key head) from the
+// float32 rows of the fused q|k|v projection, the context of a token in `splits` parts (merged by a second launch).
+struct LseFewAttention {
+  int dtype, T, H, KVH, page_tokens, splits;
+  float scale;
+  const float* qkv;         // [T, (H + 2 KVH) 64]
+  void* out;                // [T, H 64] of dtype
+  float* parts;             // splits > 1: lse_few_attention_floats()
+  void *k_pages, *v_pages;  // [pages, KVH, page_tokens, 64] of dtype
+  const float *cos, *sin;   // [positions, 32] or null
+  const int *block_tables, *ctx_lens, *cu_q, *decode_seqs;  // as in LseAttnArgs
+  int table_stride;
+};
+size_t lse_few_attention_floats(int T, int H, int splits);
+int lse_few_attention(const LseFewAttention* a, cudaStream_t stream);
+
 // out[T, N] = value of the fixed-point sums acc[T, N] (+ what out holds, if add != 0); every
 // element of acc that is read is set to zero. out float32 or bfloat16 (add needs float32).
 int lse_fixed_to_float(void* acc, void* out, int out_dtype, int add, long long n, cudaStream_t stream);

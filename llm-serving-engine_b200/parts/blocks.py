@@ -40,6 +40,9 @@ import torch
 
 from .base import (BLOCKS, FEED_FORWARDS, INPUT_FILTERS, MIXERS, NORMS, Block, PendingAdds, PendingNormedBranch,
                    count_states, flatten_needs, has_pages, settle)
+from .attention import PagedAttention
+from .feed_forward import SwiGLU
+from .norms import RMSNorm
 
 
 @dataclass(frozen=True)
@@ -66,8 +69,43 @@ class PreNormBlock(Block):
         self.mixer = self.children["mixer"]
         self.norm_post = self.children.get("norm_post")
         self.feed_forward = self.children.get("feed_forward")
+        # a layer that a kernel set may run in a few launches for few single tokens
+        self.plain = (hasattr(self.ops, "serves_few_tokens") and type(self.mixer) is PagedAttention
+                      and type(self.feed_forward) is SwiGLU and self.feed_forward.spec.activation == "silu"
+                      and not self.mixer.extended and not self.mixer.spec.bias and not self.mixer.o_bias_on
+                      and self.mixer.spec.window == 0
+                      and all(type(n) is RMSNorm and n.spec.groups == 1 for n in (self.norm_in, self.norm_post)))
+
+    def _few_tokens(self, step, cache):
+        """The step's work lists, if it is one of few single tokens that the kernel set runs in five launches a layer."""
+        T = step.num_tokens
+        if not self.plain or T > self.ops.few_tokens_max or not cache.writes:
+            return None
+        s = self.mixer.spec
+        plan = step.plans[self.mixer.plan_key()]
+        if int(plan["tiles"].shape[0]) or int(plan["decode_seqs"].shape[0]) != T:
+            return None
+        return plan if self.ops.serves_few_tokens(self.env.dtype, T, s.hidden_size, s.num_heads, s.num_kv_heads, s.head_dim,
+                                                  self.feed_forward.spec.intermediate_size) else None
+
+    def _forward_few(self, x, pending, step, cache, plan):
+        ops, m, s = self.ops, self.mixer, self.mixer.spec
+        if hasattr(pending, "resolve"):
+            pending = pending.resolve()
+        if pending is not None:
+            x = x.add_(pending)
+        cos, sin = m.rotary if m.rotary is not None else (None, None)
+        qkv = ops.norm_project(x, self.norm_in.weight, self.norm_in.spec.eps, m.qkv_weight)
+        o = ops.attend_rows(qkv, num_heads=s.num_heads, num_kv_heads=s.num_kv_heads, scale=s.scale, cos=cos, sin=sin,
+                            k_pages=cache.k, v_pages=cache.v, block_tables=step.block_tables[cache.group], step=step, plan=plan)
+        x = ops.project_rows(o, m.o_weight, x)
+        a = ops.norm_project(x, self.norm_post.weight, self.norm_post.spec.eps, self.feed_forward.gate_up_weight, pair=True)
+        return ops.project_rows(a, self.feed_forward.down_weight, x), None
 
     def forward(self, x, pending, step, cache):
+        plan = self._few_tokens(step, cache)
+        if plan is not None:
+            return self._forward_few(x, pending, step, cache, plan)
         h = self.norm_in.forward(x, settle(pending, self.norm_in))
         if getattr(self.mixer, "accepts_residual", False):
             a = self.mixer.forward(h, step, cache, residual=x, may_defer=True)  # None: already added into x

@@ -827,3 +827,84 @@ def test_unsupported_head_size_is_refused(ops):
         ops.check_attention_shape(40, torch.bfloat16)
     with pytest.raises(ValueError, match="head size"):
         ops.check_attention_shape(512, torch.float32)
+
+
+# ---------------------------------------------------------------------------- a layer of few tokens in five launches
+@pytest.mark.parametrize("dtype,T,K,N", [
+    # float32: K's slices of 8 and 16 elements, partly empty ones, the widest normed row; features that end inside a block
+    ("float32", 1, 4, 1), ("float32", 3, 100, 7), ("float32", 8, 576, 65), ("float32", 5, 1024, 24), ("float32", 2, 2052, 9),
+    # bfloat16: fewer chunks of 32 than warps, one more than they share, the widest normed row, one and two sets of tokens
+    ("bfloat16", 1, 32, 1), ("bfloat16", 8, 288, 12), ("bfloat16", 9, 800, 65), ("bfloat16", 16, 1024, 40),
+    ("bfloat16", 7, 1536, 9), ("bfloat16", 16, 4096, 8),
+])
+def test_products_of_few_tokens(ops, dtype, T, K, N):
+    """norm + product, norm + gate|up + SiLU, and product + residual add against float64. float32: K additions of
+    products around one and the norm's sum, a few 1e-7 of the result's size each. bfloat16: the activations are
+    rounded once (2^-9 of each, random: far less of a sum), the gated result once more."""
+    dt, bf16 = DT[dtype], dtype == "bfloat16"
+    x, r = rnd(T, K, seed=1, scale=2.0), rnd(T, N, seed=2)
+    nw = 1 + rnd(K, seed=3, scale=0.1)
+    w, w2 = rnd(N, K, dtype=dt, seed=4, scale=K**-0.5), rnd(2 * N, K, dtype=dt, seed=5, scale=K**-0.5)
+    a = rnd(T, K, dtype=dt, seed=6)
+    d = torch.float64
+    h = x.to(d) * torch.rsqrt((x.to(d) ** 2).mean(-1, keepdim=True) + 1e-5) * nw.to(d)
+    par = lambda t: torch.nn.Parameter(t.cuda(), requires_grad=False)
+    kw = dict(atol32=2e-6, rel16=0.01)
+    wide = K > 1024  # wider rows are not normed here
+    assert ops.ext.few_tokens_serves(bf16, T, N, K, True, False) == (not wide)
+    if not wide:
+        close(ops.norm_project(x.cuda(), nw.cuda(), 1e-5, par(w)), h @ w.to(d).T, dtype, **kw)
+        gate, up = (h @ w2.to(d).T).split(N, 1)
+        got = ops.norm_project(x.cuda(), nw.cuda(), 1e-5, w2.cuda(), pair=True)  # (no parameter: read after the wait)
+        assert got.dtype == dt
+        close(got, gate / (1 + torch.exp(-gate)) * up, dtype, **kw)
+    xg = r.cuda()
+    got = ops.project_rows(a.cuda(), par(w), xg)
+    close(got, r.to(d) + a.to(d) @ w.to(d).T, dtype, atol32=2e-6, rel16=1e-5 if K < 4096 else 2e-5)
+    assert torch.equal(xg.cpu(), r), "the residual stream is left as it was"
+    if not bf16:  # the same additions as the product of any number of rows
+        plain = torch.empty(T, N, device="cuda")
+        ops.ext.gemm_f32(a.cuda(), w.cuda(), None, plain, False)
+        assert torch.equal(ops.project_rows(a.cuda(), par(w), torch.zeros_like(xg)), plain)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("nq,nk,page,rope,splits", [(4, 4, 16, True, 0), (6, 2, 8, True, 1), (4, 1, 64, False, 60), (3, 1, 7, True, 17)])
+def test_rotation_cache_write_and_attention_from_rows_of_the_projection(ops, dtype, nq, nk, page, rope, splits):
+    """Contexts from the new token alone over whole and started tiles of keys to several rounds of tiles per warp, in one
+    part and in parts of which some have no key; every page position that was not written holds huge values."""
+    ctx_lens, D, dt = [1, 2, 16, 17, 33, 129, 1030, 8], 64, DT[dtype]
+    n = len(ctx_lens)
+    _, kp, vp, tables, positions, token_seq, step = paged_case(n, [1] * n, ctx_lens, nq, nk, D, page, dt, seed=nq + page)
+    qkv = rnd(n, (nq + 2 * nk) * D, seed=9)
+    ang = torch.outer(torch.arange(1040, dtype=torch.float64), 1.0 / (1e4 ** (torch.arange(0, D, 2, dtype=torch.float64) / D)))
+    cos, sin = (ang.cos().float(), ang.sin().float()) if rope else (None, None)
+    plain, kp_ref, vp_ref = PlainOps(), kp.clone(), vp.clone()
+    kw = dict(num_heads=nq, num_kv_heads=nk, head_dim=D)
+    q = plain.rope_kv_write(qkv.clone(), positions=positions, token_seq=token_seq, cos=cos, sin=sin, k_pages=kp_ref,
+                            v_pages=vp_ref, block_tables=tables, page_tokens=page, out_dtype=dt, **kw)
+    ref = plain.paged_attention(q, scale=D**-0.5, window=0, k_pages=kp_ref, v_pages=vp_ref, block_tables=tables,
+                                page_tokens=page, step=step, plan=None, **kw)
+    dev = lambda t: None if t is None else t.cuda()
+    kp_g, vp_g = kp.cuda(), vp.cuda()
+    gstep = SimpleNamespace(cu_q=step.cu_q.cuda(), ctx_lens=step.ctx_lens.cuda(), decode_splits=splits, max_decode_ctx=1030)
+    plan = {"decode_seqs": torch.arange(n, dtype=torch.int32, device="cuda")}
+    got = ops.attend_rows(qkv.cuda(), num_heads=nq, num_kv_heads=nk, scale=D**-0.5, cos=dev(cos), sin=dev(sin), k_pages=kp_g,
+                          v_pages=vp_g, block_tables=dev(tables), step=gstep, plan=plan)
+    close(got, ref, dtype, rel16=0.02)
+    close(kp_g, kp_ref, dtype, atol32=1e-6, rel16=0.005)
+    close(vp_g, vp_ref, dtype, atol32=1e-6, rel16=0.005)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_steps_of_few_tokens_run_both_ways(ops, dtype):
+    """A layer's five launches beside the separate kernels, at the limits of the rule: rows, width, group, head size."""
+    serves = lambda T, W=576, H=9, G=3, D=64, I=1536: ops.serves_few_tokens(DT[dtype], T, W, H, G, D, I)
+    most = 8 if dtype == "float32" else 16
+    assert serves(1) and serves(most) and not serves(most + 1)
+    assert serves(1, 1024) and not serves(1, 2048) and not serves(1, H=10, G=2) and not serves(1, D=128)
+    try:
+        ops.use_few_tokens = False
+        assert not serves(1)
+    finally:
+        ops.use_few_tokens = True
