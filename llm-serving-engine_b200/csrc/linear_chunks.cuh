@@ -7,20 +7,23 @@
 // Three launches: E_c of every (chunk, head) side by side; the chain over the chunks, element by element, which leaves
 // F_c where E_c was; the outputs of every (chunk, head) side by side.
 //
-// Everything is float32 on the CUDA cores. Operands split into two tf32 numbers on the tensor cores (three multiplies for
-// a product) were built and dropped: relative to float64 9e-7 where this has 1.8e-7 and the recurrence, token by
-// token, had 2.1e-7 (16 heads of 128 x 128, 2048 tokens), and no faster (each split is four instructions).
+// The products are float32 products on the tensor cores (split_mma.cuh). Relative to float64, 16 heads of 128 x 128, 2048
+// tokens: 2.0e-7, where the same products on the CUDA cores had 2.2e-7 and the recurrence, token by token, 2.1e-7. Operands
+// split into two tf32 numbers were built and dropped: 9e-7, and no faster.
 //
-// What bounds it: the 16-byte reads of shared memory in the outputs (four passes each, 48 for 128 multiply-adds of a
-// warp) and the FMA units; 1.4e9 multiply-adds at these sizes are 36 us at their peak. 269 us with the recurrence ->
-// 149 us (sums 40, chain 41 from memory, outputs 106 with cold caches, overlapped). With silu, back to back, recurrence ->
-// products -> products that pass over later tokens' values and do not activate rows beyond a chunk's tokens: 2048 tokens
-// 313 -> 155 -> 167 us, 8192 tokens 1204 -> 631 -> 633, portions of 700 and 1300 tokens 311 -> 163 -> 146.
+// What bounds it: 2.0e9 multiply-adds are 29 us of the tensor cores at six products each (sums 11, outputs 18; 36 us of the
+// CUDA cores at their peak), and around them each block waits for its rows, activates them and waits for the others:
+// two blocks an SM overlap that. Rows are copied to shared memory as they lie and changed there by one copy of the
+// code: through registers, with the code inlined for each operand, instructions were what a block waited for most
+// (3.6 of 11 cycles an instruction), and the tensor cores gained nothing.
+// Back to back at these sizes: recurrence 313 us, products on the CUDA cores 150, now 124; portions of 700 tokens 72 -> 62.
+// In a model's step (with silu or rotation) the outputs take 75 us where they took 94, the sums 41 as before, the chain 19.
 #pragma once
 
 #include <type_traits>
 
 #include "common.cuh"
+#include "split_mma.cuh"
 
 namespace lse {
 namespace lac {
@@ -78,81 +81,85 @@ __device__ __forceinline__ void powers(float* pw, float d) {
 
 __device__ __forceinline__ float act(float z, int silu) { return silu ? z / (1.f + expf(-z)) : z; }
 
-// Sixty-four rows of `units` pieces of work each: fetch(row, piece) of up to B rows are in flight before put(row,
-// piece, what it fetched) of the first.
-template <int B, typename Fetch, typename Put>
-__device__ __forceinline__ void for_rows(int units, Fetch fetch, Put put) {
-  const int per = THREADS / units, t0 = threadIdx.x / units, u = threadIdx.x - t0 * units;
-  if (t0 >= per) return;
+// 64 rows of `len` columns of proj (from column `col`) are asked for, into rows `ld` apart; rows from n on are zero, and
+// so is what lies behind `len` up to a multiple of 16.
+__device__ __forceinline__ void ask(float* dst, int ld, const Args& a, const Chunk& k, int col, int len) {
+  const int units = (len + 15) / 16 * 4, per = THREADS / units, t0 = threadIdx.x / units;
+  const int i = (threadIdx.x - t0 * units) * 4;
+  if (t0 < per)
 #pragma unroll 1
-  for (int t = t0; t < L; t += B * per) {
-    decltype(fetch(0, 0)) x[B];
-#pragma unroll
-    for (int b = 0; b < B; ++b)
-      if (t + b * per < L) x[b] = fetch(t + b * per, u);
-#pragma unroll
-    for (int b = 0; b < B; ++b)
-      if (t + b * per < L) put(t + b * per, u, x[b]);
-  }
+    for (int t = t0; t < L; t += per) {
+      const bool there = t < k.n && i < len;
+      const float* src = a.proj + (there ? (size_t)(k.t0 + t) * a.stride + col + i : 0);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst + t * ld + i)),
+                   "l"(src), "r"(there ? 16 : 0));
+    }
+  asm volatile("cp.async.commit_group;\n" ::);
+}
+__device__ __forceinline__ void arrived() {
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncthreads();
 }
 
-struct Pair {
-  float4 u, v, cs, sn;
-};
-
-// 64 rows of `len` columns of proj (from column `col`) into rows `ld` apart: activated, the first `rot` columns rotated
-// (pairs half a rotation apart), row t times factor(t). Rows from n on are zero, and are not activated: the division of
-// a zero takes the slow way (a portion of 65 tokens took longer than one of 128).
-template <typename F>
-__device__ __forceinline__ void stage(float* dst, int ld, const Args& a, const Chunk& k, int col, int len, int rot, F factor) {
+// In place: n rows activated, their first `rot` columns rotated (pairs half a rotation apart, position t0 + row), row t
+// times `scale` and, counted from the last row, pw[0], pw[1], ... Rows behind them are zero and stay so. One copy of this
+// code for all operands: with the values on their way through registers and the code once per operand, a block waited
+// for instructions most of its time.
+static __device__ __noinline__ void transform(float* rows, int ld, int n, int len, int rot, int silu, const float* cos,
+                                       const float* sin, size_t pos, float scale, const float* pw) {
   const int half = rot / 2;
-  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  auto at = [&](int t, int i) {
-    return t < k.n ? *reinterpret_cast<const float4*>(a.proj + (size_t)(k.t0 + t) * a.stride + col + i) : zero;
-  };
-  auto done = [&](float4 x, float f) {
-    return make_float4(act(x.x, a.silu) * f, act(x.y, a.silu) * f, act(x.z, a.silu) * f, act(x.w, a.silu) * f);
-  };
-  auto store = [&](int t, int i, float4 x) { *reinterpret_cast<float4*>(dst + t * ld + i) = x; };
+  auto done = [&](float4 x) { return make_float4(act(x.x, silu), act(x.y, silu), act(x.z, silu), act(x.w, silu)); };
+  auto factor = [&](int t) { return pw ? scale * pw[n - 1 - t] : scale; };
   const bool whole = half % 4 == 0;  // pairs in 16-byte pieces
-  if (half > 0 && whole)
-    for_rows<2>(half / 4,
-        [&](int t, int i) {
-          const size_t tab = (size_t)(k.pos + min(t, k.n - 1)) * half + 4 * i;
-          return Pair{at(t, 4 * i), at(t, half + 4 * i), *reinterpret_cast<const float4*>(a.cos + tab),
-                      *reinterpret_cast<const float4*>(a.sin + tab)};
-        },
-        [&](int t, int i, const Pair& p) {
-          if (t >= k.n) {
-            store(t, 4 * i, zero);
-            store(t, half + 4 * i, zero);
-            return;
-          }
-          const float4 u = done(p.u, 1.f), v = done(p.v, 1.f);
-          const float f = factor(t);
-          store(t, 4 * i, make_float4((u.x * p.cs.x - v.x * p.sn.x) * f, (u.y * p.cs.y - v.y * p.sn.y) * f,
-                                      (u.z * p.cs.z - v.z * p.sn.z) * f, (u.w * p.cs.w - v.w * p.sn.w) * f));
-          store(t, half + 4 * i, make_float4((v.x * p.cs.x + u.x * p.sn.x) * f, (v.y * p.cs.y + u.y * p.sn.y) * f,
-                                             (v.z * p.cs.z + u.z * p.sn.z) * f, (v.w * p.cs.w + u.w * p.sn.w) * f));
-        });
+  if (half > 0 && whole) {
+    const int units = half / 4, per = THREADS / units, t0 = threadIdx.x / units, i = (threadIdx.x - t0 * units) * 4;
+    if (t0 < per)
+#pragma unroll 1
+      for (int t = t0; t < n; t += per) {
+        float4* pu = reinterpret_cast<float4*>(rows + t * ld + i);
+        float4* pv = reinterpret_cast<float4*>(rows + t * ld + half + i);
+        const float4 cs = *reinterpret_cast<const float4*>(cos + (pos + t) * half + i);
+        const float4 sn = *reinterpret_cast<const float4*>(sin + (pos + t) * half + i);
+        const float4 u = done(*pu), v = done(*pv);
+        const float f = factor(t);
+        *pu = make_float4((u.x * cs.x - v.x * sn.x) * f, (u.y * cs.y - v.y * sn.y) * f, (u.z * cs.z - v.z * sn.z) * f,
+                          (u.w * cs.w - v.w * sn.w) * f);
+        *pv = make_float4((v.x * cs.x + u.x * sn.x) * f, (v.y * cs.y + u.y * sn.y) * f, (v.z * cs.z + u.z * sn.z) * f,
+                          (v.w * cs.w + u.w * sn.w) * f);
+      }
+  }
   const int first = whole ? rot : 0;  // (rot is a multiple of 8 then)
-  if (first < len)
-    for_rows<8>((len - first) / 4, [&](int t, int i) { return at(t, first + 4 * i); },
-                [&](int t, int i, const float4& x) { store(t, first + 4 * i, t < k.n ? done(x, factor(t)) : zero); });
-  if (half > 0 && !whole) {  // odd sizes: rotated in place (the factor is in both of a pair)
+  if (first < len && (silu || pw || scale != 1.f)) {
+    const int units = (len - first) / 4, per = THREADS / units, t0 = threadIdx.x / units;
+    const int i = first + (threadIdx.x - t0 * units) * 4;
+    if (t0 < per)
+#pragma unroll 1
+      for (int t = t0; t < n; t += per) {
+        float4* p = reinterpret_cast<float4*>(rows + t * ld + i);
+        const float4 x = done(*p);
+        const float f = factor(t);
+        *p = make_float4(x.x * f, x.y * f, x.z * f, x.w * f);
+      }
+  }
+  if (half > 0 && !whole) {  // odd sizes: rotated behind the rest (the factor is in both of a pair)
     __syncthreads();
-    for (int idx = threadIdx.x; idx < L * half; idx += THREADS) {
+#pragma unroll 1
+    for (int idx = threadIdx.x; idx < n * half; idx += THREADS) {
       const int t = idx / half, w = idx - t * half;
-      float* row = dst + t * ld;
-      const size_t tab = (size_t)(k.pos + min(t, k.n - 1)) * half + w;
-      const float cs = a.cos[tab], sn = a.sin[tab], u = row[w], v = row[w + half];
+      float* row = rows + t * ld;
+      const size_t tab = (pos + t) * half + w;
+      const float cs = cos[tab], sn = sin[tab], u = row[w], v = row[w + half];
       row[w] = u * cs - v * sn;
       row[w + half] = v * cs + u * sn;
     }
   }
 }
+__device__ __forceinline__ void transform(float* rows, int ld, const Args& a, const Chunk& k, int len, int rot, float scale,
+                                          const float* pw = nullptr) {
+  transform(rows, ld, k.n, len, rot, a.silu, a.cos, a.sin, (size_t)k.pos, scale, pw);
+}
 
-// ---- E_c, [dv][dk]: a thread has VH x KH tiles of 4 x 4, 64 rows and columns apart
+// ---- E_c, [dv][dk]: a warp has 32 VH rows and 16 KH columns of it
 template <int VH, int KH>
 __global__ void __launch_bounds__(THREADS, 2) chunk_sums_kernel(const Args a) {
   extern __shared__ __align__(16) float smem[];
@@ -164,43 +171,55 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_sums_kernel(const Args a) {
     return;
   }
   const int h = blockIdx.y, dk = a.dk, dv = a.dv;
-  constexpr int LDK = 64 * KH, LDV = 64 * VH;  // (columns beyond dk and dv are never stored)
+  constexpr int LDK = 64 * KH + 4, LDV = 64 * VH + 4;  // (columns beyond dk and dv are never stored)
   float* ks = smem;            // [64][LDK]
   float* vs = ks + L * LDK;    // [64][LDV]
   powers(pw, a.decay[h]);
-  __syncthreads();
   pdl_wait();
-  stage(ks, LDK, a, k, (a.H + h) * dk, dk, a.rot, [&](int t) { return t < k.n ? a.key_scale * pw[k.n - 1 - t] : 0.f; });
-  stage(vs, LDV, a, k, 2 * a.H * dk + h * dv, dv, 0, [](int) { return 1.f; });
+  ask(ks, LDK, a, k, (a.H + h) * dk, dk);
+  ask(vs, LDV, a, k, 2 * a.H * dk + h * dv, dv);
+  arrived();
+  transform(ks, LDK, a, k, dk, a.rot, a.key_scale, pw);
+  transform(vs, LDV, a, k, dv, 0, 1.f);
   __syncthreads();
-  const int tv = (threadIdx.x >> 4) * 4, tk = (threadIdx.x & 15) * 4;
-  float acc[VH * 4][KH * 4];
+  const int warp = threadIdx.x >> 5, g = (threadIdx.x & 31) >> 2, q = threadIdx.x & 3;
+  const int r0 = (warp >> 2) * 32 * VH, c0 = (warp & 3) * 16 * KH;
+  float acc[2 * VH][2 * KH][4];
 #pragma unroll
-  for (int i = 0; i < VH * 4; ++i)
+  for (int i = 0; i < 2 * VH; ++i)
 #pragma unroll
-    for (int j = 0; j < KH * 4; ++j) acc[i][j] = 0.f;
-#pragma unroll 2
-  for (int t = 0; t < L; ++t) {
-    float x[VH][4], y[KH][4];
+    for (int j = 0; j < 2 * KH; ++j)
 #pragma unroll
-    for (int i = 0; i < VH; ++i) load4<float>(vs + t * LDV + 64 * i + tv, x[i]);
+      for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
+#pragma unroll 1
+  for (int t = 0; t < L; t += 16) {
+    split::B y[2 * KH];
 #pragma unroll
-    for (int j = 0; j < KH; ++j) load4<float>(ks + t * LDK + 64 * j + tk, y[j]);
+    for (int j = 0; j < 2 * KH; ++j) split::down(y[j], ks + t * LDK + c0 + 8 * j + g, LDK, q);
 #pragma unroll
-    for (int i = 0; i < VH * 4; ++i)
-#pragma unroll
-      for (int j = 0; j < KH * 4; ++j) acc[i][j] = fmaf(x[i / 4][i % 4], y[j / 4][j % 4], acc[i][j]);
+    for (int i = 0; i < 2 * VH; ++i) {
+      split::A x;
+      split::down(x, vs + t * LDV + r0 + 16 * i + g, LDV, q);
+      split::multiply_add(acc[i], x, y);
+    }
   }
   float* to = a.chunks + (k.at * a.H + h) * (size_t)dv * dk;
 #pragma unroll
-  for (int i = 0; i < VH * 4; ++i) {
-    const int r = 64 * (i / 4) + tv + i % 4;
-    if (r >= dv) continue;
+  for (int i = 0; i < 2 * VH; ++i) {
+    const bool again = split::strange(acc[i]);
 #pragma unroll
-    for (int j = 0; j < KH; ++j)
-      if (64 * j + tk < dk)
-        *reinterpret_cast<float4*>(to + (size_t)r * dk + 64 * j + tk) =
-            make_float4(acc[i][4 * j], acc[i][4 * j + 1], acc[i][4 * j + 2], acc[i][4 * j + 3]);
+    for (int j = 0; j < 2 * KH; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; e += 2) {
+        const int r = r0 + 16 * i + g + 4 * e, c = c0 + 8 * j + 2 * q;
+        if (r >= dv || c >= dk) continue;
+        float* x = acc[i][j] + e;
+        if (again) {
+          if (!split::finite(x[0])) x[0] = split::dot(vs + r, LDV, ks + c, LDK, L);
+          if (!split::finite(x[1])) x[1] = split::dot(vs + r, LDV, ks + c + 1, LDK, L);
+        }
+        *reinterpret_cast<float2*>(to + (size_t)r * dk + c) = make_float2(x[0], x[1]);
+      }
   }
 }
 
@@ -248,8 +267,19 @@ __global__ void chain_kernel(const Args a) {
   store4<float>(st, S);
 }
 
-// ---- outputs: a thread has the rows ty + 16 i and the columns tx + 16 m. Rows of q, k and F are LDK = dk + 4 floats
-// apart: the 16-byte reads of eight neighbouring columns then fall into different banks.
+// ---- outputs: a warp has 32 rows and 4 M columns of them
+// Rows of q, k and F are ld_of(dk) floats apart, zeros behind dk up to a multiple of 16.
+__host__ __device__ constexpr int ld_of(int dk) { return ((dk + 15) / 16 * 16) | 16; }
+constexpr int LDP = L + 8;
+
+// The sum of n values with weights: `sum`, unless it or one of the values is no number.
+static __device__ __noinline__ float weighted(const float* p, const float* v, int ldv, int n, float sum) {
+  bool fine = split::finite(sum);
+#pragma unroll 1
+  for (int t = 0; t < n; ++t) fine = fine && split::finite(v[t * ldv]);
+  return fine ? sum : split::dot(p, 1, v, ldv, n);
+}
+
 template <int M>
 __global__ void __launch_bounds__(THREADS, 2) chunk_outputs_kernel(const Args a) {
   extern __shared__ __align__(16) float smem[];
@@ -260,163 +290,181 @@ __global__ void __launch_bounds__(THREADS, 2) chunk_outputs_kernel(const Args a)
     pdl_wait();
     return;
   }
-  const int h = blockIdx.y, dk = a.dk, dv = a.dv, ld = dk + 4, tid = threadIdx.x;
-  constexpr int LDV = 16 * M, LDP = L + 4;
-  float* qs = smem;             // [64][ld]; then the scores, [64][LDP]
-  float* fs = qs + L * (dk > L ? ld : LDP);  // F [16 M][ld]; then k [64][ld], v [64][LDV]
+  const int h = blockIdx.y, dk = a.dk, dv = a.dv, ld = ld_of(dk), tid = threadIdx.x;
+  constexpr int LDV = 16 * M + 4, NT = M / 2;  // tiles of eight columns of a warp
+  float* qs = smem;                            // [64][ld]; then the scores, [64][LDP]
+  float* fs = qs + L * (ld > LDP ? ld : LDP);  // F [dv][ld]; then k [64][ld], v [64][LDV]
   float* ks = fs;
   float* vs = ks + L * ld;
   powers(pw, a.decay[h]);
   pdl_wait();
   const float* F = a.chunks + (k.at * a.H + h) * (size_t)dv * dk;
   {
-    const int units = dk / 4, per = THREADS / units, j0 = tid / units, i = (tid - j0 * units) * 4;
+    const int units = (dk + 15) / 16 * 4, per = THREADS / units, j0 = tid / units, i = (tid - j0 * units) * 4;
     if (j0 < per)
+#pragma unroll 1
       for (int j = j0; j < dv; j += per) {
         const uint32_t dst = (uint32_t)__cvta_generic_to_shared(fs + j * ld + i);
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(F + (size_t)j * dk + i));
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(F + (i < dk ? (size_t)j * dk + i : 0)),
+                     "r"(i < dk ? 16 : 0));
       }
   }
-  asm volatile("cp.async.commit_group;\n" ::);
-  auto one = [](int) { return 1.f; };
-  stage(qs, ld, a, k, h * dk, dk, a.rot, one);
-  asm volatile("cp.async.wait_group 0;\n" ::);
+  ask(qs, ld, a, k, h * dk, dk);
+  arrived();
+  transform(qs, ld, a, k, dk, a.rot, 1.f);
   __syncthreads();
-  const int ty = tid >> 4, tx = tid & 15;
-  float acc[4][M];
+  const int warp = tid >> 5, g = (tid & 31) >> 2, q = tid & 3;
+  const int r0 = (warp >> 2) * 32, c0 = (warp & 3) * 8 * NT;
+  float acc[2][NT][4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int m = 0; m < M; ++m) acc[i][m] = 0.f;
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
   // (columns beyond dv are sums of whatever lies there, and are never stored)
-  // Sums of more than 32 terms are sums of parts of 32 (and of 16 tokens below): a chain of 128 rounds more.
 #pragma unroll 1
-  for (int d0 = 0; d0 < dk; d0 += 32) {
-    float part[4][M];
+  for (int d = 0; d < dk; d += 16) {
+    split::B f[NT];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int j = 0; j < NT; ++j) split::along(f[j], fs + (c0 + 8 * j + g) * ld + d, q);
 #pragma unroll
-      for (int m = 0; m < M; ++m) part[i][m] = 0.f;
-    const int d1 = min(dk, d0 + 32);
-#pragma unroll 1
-    for (int d = d0; d < d1; d += 4) {
-      float q[4][4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) load4<float>(qs + (ty + 16 * i) * ld + d, q[i]);
-#pragma unroll
-      for (int m = 0; m < M; ++m) {
-        float f[4];
-        load4<float>(fs + (tx + 16 * m) * ld + d, f);
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) part[i][m] = fmaf(q[i][e], f[e], part[i][m]);
-      }
+    for (int i = 0; i < 2; ++i) {
+      split::A x;
+      split::along(x, qs + (r0 + 16 * i + g) * ld + d, ld, q);
+      split::multiply_add(acc[i], x, f);
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int m = 0; m < M; ++m) acc[i][m] += part[i][m];
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float f = pw[ty + 16 * i + 1];
+  for (int i = 0; i < 2; ++i) {
+    const bool again = split::strange(acc[i]);
+    const float f[2] = {pw[r0 + 16 * i + g + 1], pw[r0 + 16 * i + g + 9]};
 #pragma unroll
-    for (int m = 0; m < M; ++m) acc[i][m] *= f;
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int r = r0 + 16 * i + g + 8 * (e >> 1), c = c0 + 8 * j + 2 * q + (e & 1);
+        if (again && c < dv && !split::finite(acc[i][j][e])) acc[i][j][e] = split::dot(qs + r * ld, 1, fs + c * ld, 1, dk);
+        acc[i][j][e] *= f[e >> 1];
+      }
   }
   __syncthreads();  // F is used up: k and v take its place
-  stage(ks, ld, a, k, (a.H + h) * dk, dk, a.rot, [&](int) { return a.key_scale; });
-  stage(vs, LDV, a, k, 2 * a.H * dk + h * dv, dv, 0, one);
+  ask(ks, ld, a, k, (a.H + h) * dk, dk);
+  ask(vs, LDV, a, k, 2 * a.H * dk + h * dv, dv);
+  arrived();
+  transform(ks, ld, a, k, dk, a.rot, a.key_scale);
+  transform(vs, LDV, a, k, dv, 0, 1.f);
   __syncthreads();
   {
+    // Scores: a warp has 16 rows and every other one of the tiles of eight columns up to their diagonal; the two warps
+    // that issue from the same quarter of the SM have five tiles together.
+    const int m = warp < 4 ? warp >> 1 : 3 - ((warp - 4) >> 1), odd = warp & 1;
     float s[4][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int j = 0; j < 4; ++j)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
+      for (int e = 0; e < 4; ++e) s[j][e] = 0.f;
 #pragma unroll 1
-    for (int d0 = 0; d0 < dk; d0 += 32) {
-      float part[4][4];
+    for (int d = 0; d < dk; d += 16) {
+      split::A x;
+      split::along(x, qs + (16 * m + g) * ld + d, ld, q);
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) part[i][j] = 0.f;
-      const int d1 = min(dk, d0 + 32);
-#pragma unroll 1
-      for (int d = d0; d < d1; d += 4) {
-        float kc[4][4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) load4<float>(ks + (tx + 16 * j) * ld + d, kc[j]);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          float q[4];
-          load4<float>(qs + (ty + 16 * i) * ld + d, q);
-#pragma unroll
-          for (int j = 0; j <= i; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) part[i][j] = fmaf(q[e], kc[j][e], part[i][j]);
+      for (int j = 0; j < 4; j += 2) {
+        if (j > m) break;
+        split::B y[2];
+        split::along(y[0], ks + (16 * j + 8 * odd + g) * ld + d, q);
+        if (j + 1 <= m) {
+          split::along(y[1], ks + (16 * j + 16 + 8 * odd + g) * ld + d, q);
+          split::multiply_add(reinterpret_cast<float(&)[2][4]>(s[j]), x, y);
+        } else {
+          split::multiply_add(reinterpret_cast<float(&)[1][4]>(s[j]), x, reinterpret_cast<const split::B(&)[1]>(y[0]));
         }
       }
+    }
+    if (split::strange(s)) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int j = 0; j < 4; ++j)
 #pragma unroll
-        for (int j = 0; j <= i; ++j) s[i][j] += part[i][j];
+        for (int e = 0; e < 4; ++e)
+          if (j <= m && !split::finite(s[j][e]))
+            s[j][e] = split::dot(qs + (16 * m + g + 8 * (e >> 1)) * ld, 1, ks + (16 * j + 8 * odd + 2 * q + (e & 1)) * ld, 1, dk);
     }
     __syncthreads();  // q is used up
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int j = 0; j < 4; ++j)
 #pragma unroll
-      for (int j = 0; j <= i; ++j) {
-        const int back = ty + 16 * i - (tx + 16 * j);
-        qs[(ty + 16 * i) * LDP + tx + 16 * j] = back >= 0 ? s[i][j] * pw[max(back, 0)] : 0.f;
-      }
+      for (int e = 0; e < 4; e += 2)
+        if (j <= m) {
+          const int r = 16 * m + g + 4 * e, c = 16 * j + 8 * odd + 2 * q, back = r - c;
+          *reinterpret_cast<float2*>(qs + r * LDP + c) = make_float2(back >= 0 ? s[j][e] * pw[max(back, 0)] : 0.f,
+                                                                     back >= 1 ? s[j][e + 1] * pw[max(back - 1, 0)] : 0.f);
+        }
   }
   __syncthreads();
+  // Values, two tiles of columns at a time. Those that are no number are left out of the products (a later token's would
+  // be met by a zero, and be no number all the same); sums that have one are taken again.
 #pragma unroll
-  for (int b = 0; b < 4; ++b) {  // tokens of block b reach rows of the blocks i >= b
-    float part[4][M];
+  for (int j0 = 0; j0 < NT; j0 += 2) {
+    float part[2][2][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int m = 0; m < M; ++m) part[i][m] = 0.f;
-    // A later token's value is left out of the row's own block and not only met by a zero: it may be no number. A warp
-    // has two rows of each block, so four tokens are all of them before, all of them behind, or looked at one by one.
-    auto four = [&](int t, auto own) {
-      float p[4][4];
+      for (int j = 0; j < 2; ++j)
 #pragma unroll
-      for (int i = b; i < 4; ++i) load4<float>(qs + (ty + 16 * i) * LDP + t, p[i]);
+        for (int e = 0; e < 4; ++e) part[i][j][e] = 0.f;
+    bool again = false;
+#pragma unroll 1
+    for (int t = 0; t < r0 + 32; t += 16) {
+      split::B y[2];
 #pragma unroll
-      for (int m = 0; m < M; ++m)
+      for (int j = 0; j < 2; ++j) {
+        const float* p = vs + (t + 2 * q) * LDV + c0 + 8 * (j0 + j) + g;
+        float x[4] = {p[0], p[LDV], p[8 * LDV], p[9 * LDV]};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (!split::finite(x[e])) {
+            x[e] = 0.f;
+            again = again || c0 + 8 * (j0 + j) + g < dv;
+          }
+        y[j].set(0, x[0], x[1]), y[j].set(1, x[2], x[3]);
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        if (t > r0 + 16 * i) continue;
+        split::A x;
+        split::along_as_down(x, qs + (r0 + 16 * i + g) * LDP + t, LDP, q);
+        split::multiply_add(part[i], x, y);
+      }
+    }
+    again = __any_sync(0xffffffffu, again || split::strange(part[0]) || split::strange(part[1]));
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const float v = vs[(t + e) * LDV + tx + 16 * m];
-          if constexpr (own.value == 2) part[b][m] = fmaf(p[b][e], v, part[b][m]);
-          if constexpr (own.value == 1) part[b][m] = fmaf(p[b][e], t + e <= ty + 16 * b ? v : 0.f, part[b][m]);
-#pragma unroll
-          for (int i = b + 1; i < 4; ++i) part[i][m] = fmaf(p[i][e], v, part[i][m]);
+          if (again) {
+            const int r = r0 + 16 * i + g + 8 * (e >> 1), c = c0 + 8 * (j0 + j) + 2 * q + (e & 1);
+            if (c < dv) part[i][j][e] = weighted(qs + r * LDP, vs + c, LDV, r + 1, part[i][j][e]);
+          }
+          acc[i][j0 + j][e] += part[i][j][e];
         }
-    };
-    const int mixed = 16 * b + (ty & ~3);  // (the same for both rows of the warp)
-#pragma unroll 1
-    for (int t = 16 * b; t < mixed; t += 4) four(t, std::integral_constant<int, 2>());
-    four(mixed, std::integral_constant<int, 1>());
-    if (b < 3)
-#pragma unroll 1
-      for (int t = mixed + 4; t < 16 * b + 16; t += 4) four(t, std::integral_constant<int, 0>());
-#pragma unroll
-    for (int i = b; i < 4; ++i)
-#pragma unroll
-      for (int m = 0; m < M; ++m) acc[i][m] += part[i][m];
+    __syncwarp();
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int t = ty + 16 * i;
-    if (t >= k.n) continue;
-    float* to = a.out + (size_t)(k.t0 + t) * ((size_t)a.H * dv) + (size_t)h * dv + tx;
+  for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int m = 0; m < M; ++m)
-      if (tx + 16 * m < dv) to[16 * m] = acc[i][m] * a.query_scale;
-  }
+    for (int e = 0; e < 4; e += 2) {
+      const int t = r0 + 16 * i + g + 4 * e;
+      if (t >= k.n) continue;
+      float* to = a.out + (size_t)(k.t0 + t) * ((size_t)a.H * dv) + (size_t)h * dv + c0 + 2 * q;
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+        if (c0 + 8 * j + 2 * q < dv) {
+          to[8 * j] = acc[i][j][e] * a.query_scale;
+          to[8 * j + 1] = acc[i][j][e + 1] * a.query_scale;
+        }
+    }
 }
 
 // Rows of whole 16-byte pieces, and sizes whose tiles fit the shared memory.
@@ -428,15 +476,18 @@ inline bool serves(const Args& a) {
 
 template <int VH, int KH>
 inline bool launch_sums(const Args& a, dim3 grid, cudaStream_t stream) {
-  constexpr int smem = L * 64 * (VH + KH) * 4;
+  constexpr int smem = L * (64 * (VH + KH) + 8) * 4;
   return allow_dynamic_smem<chunk_sums_kernel<VH, KH>, smem>() == cudaSuccess &&
          launch(chunk_sums_kernel<VH, KH>, grid, THREADS, smem, stream, a) == cudaSuccess;
 }
 template <int M>
 inline bool launch_outputs(const Args& a, dim3 grid, cudaStream_t stream) {
-  const int ld = a.dk + 4, first = 16 * M * ld, second = L * (ld + 16 * M);
-  const int smem = (L * (a.dk > L ? ld : L + 4) + (first > second ? first : second)) * 4;
-  constexpr int most = (L * (MAX + 4) + (16 * M > L ? 16 * M * (MAX + 4) : 0) + L * (MAX + 4 + 16 * M)) * 4;
+  auto bytes = [](int ld, int dv) {
+    const int first = dv * ld, second = L * (ld + 16 * M + 4);
+    return (L * (ld > LDP ? ld : LDP) + (first > second ? first : second)) * 4;
+  };
+  constexpr int most = bytes(ld_of(MAX), 16 * M);
+  const int smem = bytes(ld_of(a.dk), 16 * M);
   return allow_dynamic_smem<chunk_outputs_kernel<M>, most>() == cudaSuccess &&
          launch(chunk_outputs_kernel<M>, grid, THREADS, smem, stream, a) == cudaSuccess;
 }

@@ -472,7 +472,7 @@ __global__ void norm_rope_kv_write_kernel(const float* __restrict__ qkv, T* __re
 // thread's rows are contiguous there.
 //
 // A portion longer than L tokens is cut into chunks of L. With a decay per head and key and value sizes that are
-// multiples of 4 up to 128 they run as matrix products (linear_chunks.cuh, 149 against 269 us at 16 heads of 128 x 128
+// multiples of 4 up to 128 they run as matrix products (linear_chunks.cuh, 124 against 313 us at 16 heads of 128 x 128
 // and 2048 tokens); otherwise side by side here, in three launches:
 //   A  every chunk steps through its tokens from a zero state (the first chunk from the request's
 //      state) and leaves its outputs and its final state (chunk c: E_c) in a scratch;

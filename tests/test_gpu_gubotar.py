@@ -172,6 +172,23 @@ def test_linear_attention_chunk_products_at_their_edges(ops, H, dk, dv, rot, sil
     assert bool((state[[4, 6]] == 1e4).all())
 
 
+@pytest.mark.parametrize("dk,dv", [(4, 4), (12, 20), (16, 8), (80, 36), (100, 128), (128, 68), (128, 128)])
+def test_linear_attention_chunk_products_are_float32_products(ops, dk, dv):
+    """Rows of magnitudes 2^-12 to 2^12 beside one another, at sizes around the tiles of 8 and 16. A sum of up to 128
+    products is within 2^-22 (what three parts of each number leave out) and 16 roundings of 2^-24 of the sum of the
+    products' absolute values; three such products follow one another, and the powers of the decay add less than one."""
+    H, n = 2, 141
+    decay = [0.99, 0.6]
+    proj = rnd(n, 2 * H * dk + H * dv, seed=dk) * 2.0 ** torch.randint(-12, 13, (n, 1), generator=torch.Generator().manual_seed(3))
+    state = torch.zeros(1, H, dv, dk).cuda()
+    got = ops.decay_linear_attention(proj.cuda(), num_heads=H, key_dim=dk, value_dim=dv, decay=torch.tensor(decay).cuda(),
+                                     activation="none", key_scale=dk ** -0.5, cos=None, sin=None, state=state,
+                                     step=batch([n], [0], [0]))
+    decay = torch.tensor(decay).double().tolist()
+    ref, size = (linear_attention_reference(x, H, dk, dv, decay, False, 0, 0, dk ** -0.5) for x in (proj, proj.abs()))
+    assert bool(((got.double().cpu() - ref).abs() <= 4 * (2.0 ** -22 + 16 * 2.0 ** -24) * size).all())
+
+
 @pytest.mark.parametrize("products", [False, True])
 @pytest.mark.parametrize("lens", [[65], [128, 129], [60, 80, 1], [64, 200, 33]])
 def test_linear_attention_either_way_of_running_chunks(ops, monkeypatch, lens, products):
