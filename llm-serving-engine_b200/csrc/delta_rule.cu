@@ -15,6 +15,7 @@
 // sequence whose first row of this step is at position 0 starts from zeros whatever its slot holds.
 #include "common.cuh"
 #include "kernels.h"
+#include "split_mma.cuh"
 
 namespace lse {
 
@@ -475,7 +476,7 @@ __global__ void __launch_bounds__(DR_THREADS) delta_rule_kernel(const DeltaRule 
 //   B  per head and slice of DC_B columns, chunk after chunk: u = U - S0 W and the next S0 (the states
 //      before each chunk are kept);
 //   C  per chunk, head and slice of columns, side by side: the outputs.
-// All in float32 (register-tiled products on the CUDA cores); the decays enter as products of
+// All in float32 (A and C: register-tiled products on the CUDA cores, B: split_mma.cuh); the decays enter as products of
 // factors in (0, 1], so nothing overflows. A chunk that is not full is filled up with tokens of
 // g = 1, beta = 0 and zero vectors.
 //
@@ -497,7 +498,6 @@ struct DeltaChunks {
   int H, G, dk, dv;
   int ld;              // row length of q, k, W and state rows: dk up to a multiple of 16, + 4 (zeros behind dk)
   int dvp;             // dv up to a multiple of DC_B
-  int stages;          // launch B: chunks staged at a time
   // scratch per (chunk, head), laid out as the kernels stage it
   float* wk;           // [2][64][ld]: W, then r_(last,t) k_t
   float* u;            // [dvp / 16][64][16]: U, then u, in the slices of launch B
@@ -977,11 +977,29 @@ __global__ void __launch_bounds__(DC_THREADS, 2) delta_channel_systems_kernel(co
 }
 
 // ---- launch B
-template <bool CH>
-__global__ void __launch_bounds__(DC_B_THREADS) delta_chunk_states_kernel(const DeltaChunks a) {
-  extern __shared__ __align__(16) float dc_smem[];
+// A block has DC_B columns of a head's state and goes through the chunks one after another. Both products are float32
+// products on the tensor cores (split_mma.cuh), transposed: rows are the block's 16 columns of the state.
+//   u^T [16 x 64]   = U^T - S [16 x dk] W^T     a warp has eight tokens (its columns of W^T are its own)
+//   S   [16 x dk]   = G S + u^T [16 x 64] (r k) a warp has 16 key dims, 128 and more on again, and keeps them
+// S stays in the accumulators' registers. What one warp makes and all need, S and u^T, is cut into its three parts by
+// the lane that made it and passed on through shared memory as operand registers; what one warp alone needs, its part of
+// W and of r k, comes from memory straight into registers, a chunk ahead.
+// Which of the sixteen terms of a product a lane has, and which key dim is which column of its tiles, is chosen so that
+// nothing changes lanes: lane 4 g + q holds the key dims 4 q .. 4 q + 3 of the columns g and g + 8.
+//
+// What bounds it: the chain of chunks, 2 us each: 97 products a warp in two rounds with a barrier behind each, and two
+// warps to a scheduler, so that the latencies of cutting operands and of the tensor cores show. With 128 registers, for
+// two blocks an SM, some of what is fetched ahead is spilled, and a spill waits for its number: 3.9 us a chunk.
+// On the CUDA cores (staged in shared memory; 5 us a chunk and block) its reads were the bound: 3.1 passes each.
+// Portions of 666 and 1333 tokens, 16 heads of 128 x 128: 160 -> 120 us. All three launches, 2048 tokens: 304 -> 269 us with a
+// decay per channel, 257 -> 240 per head; 700 tokens 118 -> 106, 101 -> 92. Relative to float64: outputs 3.6e-7 -> 3.4e-7, state
+// 2.8e-7 -> 2.5e-7 with slow decays; where a state is its last two or three tokens, 0.9e-7 -> 1.0e-7.
+template <bool CH, int NB>  // NB: dk up to 128 NB
+__global__ void __launch_bounds__(DC_B_THREADS, 1) delta_chunk_states_kernel(const DeltaChunks a) {
+  __shared__ uint4 s_parts[3][8 * NB][32];  // S, cut: operand registers of every lane per sixteen key dims
+  __shared__ __align__(16) uint2 u_parts[3][DC_L / 16][32][2];
   pdl_trigger();
-  const int dk = a.dk, dv = a.dv, ld = a.ld, tid = threadIdx.x;
+  const int dk = a.dk, dv = a.dv, ld = a.ld, kd = ld - 4;
   const int slices = a.dvp / DC_B;
   const int h = blockIdx.x / slices, slice = blockIdx.x - h * slices, c0 = slice * DC_B, seq = blockIdx.y;
   const int r0 = a.cu_q[seq], n = a.cu_q[seq + 1] - r0;
@@ -990,131 +1008,166 @@ __global__ void __launch_bounds__(DC_B_THREADS) delta_chunk_states_kernel(const 
     return;
   }
   const int chunks = (n + DC_L - 1) / DC_L;
-  const int cols = min(DC_B, dv - c0);
   const size_t first = (size_t)dc_first_chunk(a.cu_q, seq) * a.H + h;
-  const int per = DC_L * (2 * ld + DC_B);  // a staged chunk: W, r k [64][ld] each, U [64][16]
-  float* Ss = dc_smem + a.stages * per;    // [16][ld]: the state's columns
-  float* part = Ss + DC_B * ld;            // sums of parts: [8][64][20] in the first product, [8][16][32] in the second
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  const int d0 = 16 * warp + 4 * q;  // + 128 b: this lane's four key dims
   pdl_wait();
-  auto issue = [&](int c, float* ws) {
+
+  float4 w[8 * NB];          // W of token 8 warp + g: key dims 16 k + 4 q ..
+  float2 rk[NB][DC_L / 16][4];  // r k of tokens 16 s + 2 q + {0, 1, 8, 9}: key dims 16 warp + 2 g, + 1
+  float uu[4];               // U of tokens 8 warp + 2 q, + 1, column g; then column g + 8
+  auto fetch_w = [&](int c) {
     const size_t at = first + (size_t)c * a.H;
-    dc_stage_flat<DC_B_THREADS>(ws, a.wk + at * 2 * DC_L * ld, 2 * DC_L * ld);
-    dc_stage_flat<DC_B_THREADS>(ws + 2 * DC_L * ld, a.u + at * DC_L * a.dvp + (size_t)c0 * DC_L, DC_L * DC_B);
-    asm volatile("cp.async.commit_group;\n" ::);
+    const float* p = a.wk + at * 2 * DC_L * ld + (8 * warp + g) * ld + 4 * q;
+#pragma unroll
+    for (int k = 0; k < 8 * NB; ++k)
+      if (16 * k < kd) w[k] = *reinterpret_cast<const float4*>(p + 16 * k);
+    const float* u = a.u + at * DC_L * a.dvp + (size_t)c0 * DC_L + (8 * warp + 2 * q) * DC_B + g;
+    uu[0] = u[0], uu[1] = u[DC_B], uu[2] = u[8], uu[3] = u[DC_B + 8];
   };
-  issue(0, dc_smem);
+  auto fetch_rk = [&](int c) {
+    const float* p = a.wk + ((first + (size_t)c * a.H) * 2 + 1) * DC_L * ld + 2 * q * ld + 16 * warp + 2 * g;
+#pragma unroll
+    for (int b = 0; b < NB; ++b)
+      if (16 * warp + 128 * b < kd)
+#pragma unroll
+        for (int s = 0; s < DC_L / 16; ++s)
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            rk[b][s][e] = *reinterpret_cast<const float2*>(p + (16 * s + (e & 1) + 8 * (e >> 1)) * ld + 128 * b);
+  };
+  fetch_w(0);
+
+  float S[NB][2][4];  // columns g, g + 8; key dims d0 ..
   float* st = a.state + (((size_t)a.slots[seq] * a.H + h) * dv + c0) * dk;
   const bool read = a.ctx_lens[seq] - n > 0;
-  for (int j = tid >> 5; j < DC_B; j += DC_B_THREADS / 32)
-    for (int d = tid & 31; d < ld; d += 32)
-      Ss[j * ld + d] = (read && j < cols && d < dk) ? __ldcg(st + (size_t)j * dk + d) : 0.f;
-  // first product: a warp has an eighth of the key dims, its lanes rows rg + 8 i and columns cg + 4 j
-  const int warp = tid >> 5, cg = tid & 3, rg = (tid & 31) >> 2;
-  const int eighth = ((ld - 4) / 4 + 7) / 8 * 4, d0 = min(warp * eighth, ld - 4), d1 = min(d0 + eighth, ld - 4);
-  // second product: a warp covers 32 key dims x 16 columns (tiles of four x four) and a part of the rows
-  const int dims = (ld - 4 + 31) / 32;
-  const int parts = dims == 1 ? 8 : dims == 2 ? 4 : dims <= 4 ? 2 : 1;
-  const int tpart = warp / dims, trows = DC_L / parts;
-  const int td = (warp - tpart * dims) * 32 + (tid & 7) * 4, tj = ((tid >> 3) & 3) * 4;
+#pragma unroll
+  for (int b = 0; b < NB; ++b)
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int col = g + 8 * r, d = d0 + 128 * b + e;
+        S[b][r][e] = read && c0 + col < dv && d < dk ? __ldcg(st + (size_t)col * dk + d) : 0.f;
+      }
+  // the state before chunk c: for launch C, and for the next product
+  auto hand_on = [&](int c) {
+    float* s0 = a.s0 + ((first + (size_t)c * a.H) * a.dvp + c0) * ld;
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      if (16 * warp + 128 * b >= kd) continue;
+      split::A x;
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        store4<float>(s0 + (size_t)(g + 8 * r) * ld + d0 + 128 * b, S[b][r]);
+        x.set(r, S[b][r][0], S[b][r][1]);
+        x.set(2 + r, S[b][r][2], S[b][r][3]);
+      }
+      s_parts[0][8 * b + warp][lane] = make_uint4(x.h[0], x.h[1], x.h[2], x.h[3]);
+      s_parts[1][8 * b + warp][lane] = make_uint4(x.m[0], x.m[1], x.m[2], x.m[3]);
+      s_parts[2][8 * b + warp][lane] = make_uint4(x.l[0], x.l[1], x.l[2], x.l[3]);
+    }
+  };
+  auto part = [](uint32_t (&to)[4], const uint4& x) { to[0] = x.x, to[1] = x.y, to[2] = x.z, to[3] = x.w; };
+  hand_on(0);
+  __syncthreads();
   for (int c = 0; c < chunks; ++c) {
-    float* ws = dc_smem + (a.stages > 1 ? (c & 1) * per : 0);
-    if (a.stages > 1 && c + 1 < chunks) {
-      issue(c + 1, dc_smem + ((c + 1) & 1) * per);
-      asm volatile("cp.async.wait_group 1;\n" ::);
-    } else {
-      asm volatile("cp.async.wait_group 0;\n" ::);
-    }
-    __syncthreads();
-    const float* ks = ws + DC_L * ld;
-    float* us = ws + 2 * DC_L * ld;
     const size_t at = first + (size_t)c * a.H;
-    const float whole = CH ? 1.f : __ldg(a.g + at * DC_L + DC_L - 1);
-    dc_store_flat<DC_B_THREADS>(a.s0 + (at * a.dvp + c0) * ld, Ss, DC_B * ld);
-    float acc[8][4];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-    for (int d = d0; d < d1; d += 4) {
-      float4 s[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) s[j] = *reinterpret_cast<const float4*>(Ss + (cg + 4 * j) * ld + d);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float4 w = *reinterpret_cast<const float4*>(ws + (rg + 8 * i) * ld + d);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          acc[i][j] = fmaf(w.x, s[j].x, acc[i][j]);
-          acc[i][j] = fmaf(w.y, s[j].y, acc[i][j]);
-          acc[i][j] = fmaf(w.z, s[j].z, acc[i][j]);
-          acc[i][j] = fmaf(w.w, s[j].w, acc[i][j]);
-        }
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) part[(warp * DC_L + rg + 8 * i) * 20 + cg + 4 * j] = acc[i][j];
-    __syncthreads();
     {
-      const int t = tid >> 2, q = 4 * (tid & 3);
-      float4 u = *reinterpret_cast<const float4*>(us + t * DC_B + q);
+      float acc[4] = {0.f, 0.f, 0.f, 0.f}, low[2][4] = {};
 #pragma unroll
-      for (int g = 0; g < 8; ++g) {
-        const float4 v = *reinterpret_cast<const float4*>(part + (g * DC_L + t) * 20 + q);
-        u.x -= v.x; u.y -= v.y; u.z -= v.z; u.w -= v.w;
-      }
-      *reinterpret_cast<float4*>(us + t * DC_B + q) = u;
-    }
-    __syncthreads();
-    dc_store_flat<DC_B_THREADS>(a.u + at * DC_L * a.dvp + (size_t)c0 * DC_L, us, DC_L * DC_B);
-    if (tpart < parts) {
-      float s[4][4];  // [column][dim]
+      for (int k = 0; k < 8 * NB; k += 2) {
+        if (k == 4 * NB) fetch_rk(c);  // (half of W's registers are free by then)
+        if (16 * k >= kd) continue;
+        split::A x[2];
+        split::B y[2];
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) s[j][e] = 0.f;
-      const float* kp = ks + tpart * trows * ld + min(td, ld - 4);  // (dims beyond the row's: the zeros behind it)
-      const float* up = us + tpart * trows * DC_B + tj;
-#pragma unroll 8
-      for (int t = 0; t < trows; ++t, kp += ld, up += DC_B) {
-        const float4 k = *reinterpret_cast<const float4*>(kp);
-        const float4 v = *reinterpret_cast<const float4*>(up);
-        const float vv[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          s[j][0] = fmaf(k.x, vv[j], s[j][0]);
-          s[j][1] = fmaf(k.y, vv[j], s[j][1]);
-          s[j][2] = fmaf(k.z, vv[j], s[j][2]);
-          s[j][3] = fmaf(k.w, vv[j], s[j][3]);
+        for (int v = 0; v < 2; ++v) {
+          const bool there = v == 0 || 16 * (k + 1) < kd;
+          const float4 z = there ? w[k + v] : make_float4(0.f, 0.f, 0.f, 0.f);
+          y[v].set(0, z.x, z.y), y[v].set(1, z.z, z.w);
+          const int kk = there ? k + v : k;
+          part(x[v].h, s_parts[0][kk][lane]), part(x[v].m, s_parts[1][kk][lane]), part(x[v].l, s_parts[2][kk][lane]);
         }
+        split::multiply_add_terms(acc, low, x, y);
+      }
+      const float* s0 = a.s0 + (at * a.dvp + c0) * ld;
+      float* u = a.u + at * DC_L * a.dvp + (size_t)c0 * DC_L + (8 * warp + 2 * q) * DC_B + g;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[e] += low[0][e] + low[1][e];
+      const bool again = split::strange(reinterpret_cast<const float(&)[1][4]>(acc));
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (again && !split::finite(acc[e]))
+          acc[e] = split::dot(a.wk + at * 2 * DC_L * ld + (8 * warp + 2 * q + (e & 1)) * ld, 1,
+                              s0 + (size_t)(g + 8 * (e >> 1)) * ld, 1, dk);
+        acc[e] = uu[e] - acc[e];
+        u[(e & 1) * DC_B + 8 * (e >> 1)] = acc[e];
+      }
+      uint32_t hi[2], mid[2], rest[2];
+      split::cut(acc[0], acc[1], hi[0], mid[0], rest[0]);
+      split::cut(acc[2], acc[3], hi[1], mid[1], rest[1]);
+      u_parts[0][warp >> 1][lane][warp & 1] = make_uint2(hi[0], hi[1]);
+      u_parts[1][warp >> 1][lane][warp & 1] = make_uint2(mid[0], mid[1]);
+      u_parts[2][warp >> 1][lane][warp & 1] = make_uint2(rest[0], rest[1]);
+    }
+    const bool more = c + 1 < chunks;
+    __syncthreads();
+    if (16 * warp >= kd && more) fetch_w(c + 1);
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      if (16 * warp + 128 * b >= kd) continue;
+      float acc[2][4] = {}, low[2][4] = {}, G[4];  // G: the chunk's decay of the lane's key dims
+      if constexpr (CH) load4<float>(a.g + at * ld + d0 + 128 * b, G);
+      else G[0] = G[1] = G[2] = G[3] = a.g[at * DC_L + DC_L - 1];
+#pragma unroll
+      for (int s = 0; s < DC_L / 16; ++s) {
+        if (b == 0 && s == 2 && more) fetch_w(c + 1);
+        split::A x;
+        part(x.h, *reinterpret_cast<const uint4*>(u_parts[0][s][lane]));
+        part(x.m, *reinterpret_cast<const uint4*>(u_parts[1][s][lane]));
+        part(x.l, *reinterpret_cast<const uint4*>(u_parts[2][s][lane]));
+        split::B y[2];
+        const float2* z = rk[b][s];
+        y[0].set(0, z[0].x, z[1].x), y[0].set(1, z[2].x, z[3].x);
+        y[1].set(0, z[0].y, z[1].y), y[1].set(1, z[2].y, z[3].y);
+        split::multiply_add(acc, low, x, y);
+      }
+      // column 2 q + v of tile j is key dim 4 q + 2 v + j
+      if (split::strange(acc) || split::strange(low)) {
+        const float* k = a.wk + (at * 2 + 1) * DC_L * ld + d0 + 128 * b;
+        const float* u = a.u + at * DC_L * a.dvp + (size_t)c0 * DC_L + g;
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (!split::finite(acc[j][e]) || !split::finite(low[j][e])) {
+              acc[j][e] = split::dot(k + 2 * (e & 1) + j, ld, u + 8 * (e >> 1), DC_B, DC_L);
+              low[j][e] = 0.f;
+            }
       }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) store4<float>(part + (warp * DC_B + tj + j) * 32 + (tid & 7) * 4, s[j]);
+      for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int i = 2 * r + (e >> 1);
+          S[b][r][e] = fmaf(S[b][r][e], G[e], low[e & 1][i]) + acc[e & 1][i];
+        }
     }
-    __syncthreads();
-    for (int b = tid >> 7; b < dims; b += 2) {
-      const int j = (tid >> 3) & 15, d = b * 32 + (tid & 7) * 4;
-      if (d >= ld - 4) continue;
-      float4* p = reinterpret_cast<float4*>(Ss + j * ld + d);
-      float4 o = *p;
-      if constexpr (CH) {
-        const float4 w = __ldg(reinterpret_cast<const float4*>(a.g + at * ld + d));
-        o.x *= w.x; o.y *= w.y; o.z *= w.z; o.w *= w.w;
-      } else {
-        o.x *= whole; o.y *= whole; o.z *= whole; o.w *= whole;
-      }
-      for (int g = 0; g < parts; ++g) {
-        const float4 v = *reinterpret_cast<const float4*>(part + ((g * dims + b) * DC_B + j) * 32 + (tid & 7) * 4);
-        o.x += v.x; o.y += v.y; o.z += v.z; o.w += v.w;
-      }
-      *p = o;
+    if (more) {
+      hand_on(c + 1);
+      __syncthreads();
     }
-    __syncthreads();  // the state is whole, and the staged chunk is free
-    if (a.stages == 1 && c + 1 < chunks) issue(c + 1, dc_smem);
   }
-  for (int j = tid >> 5; j < cols; j += DC_B_THREADS / 32)
-    for (int d = tid & 31; d < dk; d += 32) st[(size_t)j * dk + d] = Ss[j * ld + d];
+#pragma unroll
+  for (int b = 0; b < NB; ++b)
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int col = g + 8 * r, d = d0 + 128 * b + e;
+        if (c0 + col < dv && d < dk) st[(size_t)col * dk + d] = S[b][r][e];
+      }
 }
 
 // ---- launch C
@@ -1335,13 +1388,10 @@ static int launch_delta_chunks(const DeltaRule& r, int num_seqs, int max_chunks,
   if (r.H > 65535 || max_chunks > 65535) return LSE_BAD_ARGUMENT;
   const size_t smem_a = CH ? channel_systems_floats(a.ld, a.dvp) * sizeof(float) :
       (size_t)(DC_L * a.ld + DC_L * (a.ld > a.dvp ? a.ld : a.dvp) + DC_L * DC_LDP + 4 * DC_L) * sizeof(float);
-  const size_t per = (size_t)DC_L * (2 * a.ld + DC_B), rest = (size_t)DC_B * a.ld + 8 * DC_L * 20;
-  a.stages = (2 * per + rest) * sizeof(float) <= 227 * 1024 ? 2 : 1;
-  const size_t smem_b = (a.stages * per + rest) * sizeof(float);
   size_t smem_c = (size_t)2 * DC_L * a.ld * sizeof(float);
   const size_t second = (size_t)DC_L * (DC_LDP + DC_N) * sizeof(float);  // what the second product stages in the same place
   if (smem_c < second) smem_c = second;
-  if (!allow_smem<delta_chunk_states_kernel<CH>>(smem_b) || !allow_smem<delta_chunk_outputs_kernel<CH>>(smem_c))
+  if (!allow_smem<delta_chunk_outputs_kernel<CH>>(smem_c))
     return LSE_LAUNCH_FAILED;
   const dim3 grid_a(max_chunks, r.H, num_seqs);
   if constexpr (CH) {
@@ -1360,7 +1410,8 @@ static int launch_delta_chunks(const DeltaRule& r, int num_seqs, int max_chunks,
     if (!allow_smem<delta_chunk_systems_kernel>(smem_a)) return LSE_LAUNCH_FAILED;
     launch(delta_chunk_systems_kernel, grid_a, DC_THREADS, smem_a, stream, a);
   }
-  launch(delta_chunk_states_kernel<CH>, dim3(r.H * (a.dvp / DC_B), num_seqs), DC_B_THREADS, smem_b, stream, a);
+  launch(a.ld - 4 <= 128 ? delta_chunk_states_kernel<CH, 1> : delta_chunk_states_kernel<CH, 2>,
+         dim3(r.H * (a.dvp / DC_B), num_seqs), DC_B_THREADS, 0, stream, a);
   const int slices = r.H * ((r.dv + DC_N - 1) / DC_N);
   if (slices > 65535) return LSE_BAD_ARGUMENT;
   launch(delta_chunk_outputs_kernel<CH>, dim3(max_chunks, slices, num_seqs), DC_THREADS, smem_c, stream, a);

@@ -8,7 +8,7 @@
 // F_c where E_c was; the outputs of every (chunk, head) side by side.
 //
 // The products are float32 products on the tensor cores (split_mma.cuh). Relative to float64, 16 heads of 128 x 128, 2048
-// tokens: 2.0e-7, where the same products on the CUDA cores had 2.2e-7 and the recurrence, token by token, 2.1e-7. Operands
+// tokens: 1.6e-7, where the same products on the CUDA cores had 2.2e-7 and the recurrence, token by token, 2.1e-7. Operands
 // split into two tf32 numbers were built and dropped: 9e-7, and no faster.
 //
 // What bounds it: 2.0e9 multiply-adds are 29 us of the tensor cores at six products each (sums 11, outputs 18; 36 us of the

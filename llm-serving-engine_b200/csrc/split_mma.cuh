@@ -1,11 +1,12 @@
 // Products of float32 matrices on the tensor cores, as exact as on the CUDA cores.
 //
-// A float32 number has 24 bits: cut off after 8 and after 16 it is the sum of three bfloat16 numbers, h + m + l, without
-// a remainder. Of the nine products of two such sums six are taken (h h, h m, m h, h l, l h, m m; each is exact in
-// float32); the other three together are below 2^-22 of the product, 2^-25 on average. The tensor cores add sixteen
-// products and cut the sum off (they do not round it), so a sum must not run on in them for long: the products of
-// sixteen terms are chained from zero, and their sum is added to a float32 accumulator by the CUDA cores. 1017 multiply-adds a clock and SM / 6 = 170, where the CUDA cores have 126 at best, and what counts more: a
-// warp's tile of 32 x 32 reads 16 numbers of shared memory for 128 multiply-adds of a lane.
+// A float32 number has 24 bits: rounded to bfloat16 (8 bits), and what is left rounded to bfloat16, it is the sum of
+// three such numbers, h + m + l, without a remainder. Of the nine products of two such sums six are taken (h h, h m, m h,
+// h l, l h, m m; each is exact in float32); the other three together are below 2^-25 of the product. The tensor cores
+// add sixteen products and cut the sum off (they do not round it), so a sum must not run on in them for long: the
+// products h h of sixteen terms, which hardly lose a bit, are summed from zero and added to a float32 accumulator by the
+// CUDA cores, as is the sum of the others. 1017 multiply-adds a clock and SM / 6 = 170, where the CUDA cores have 126 at
+// best, and what counts more: a warp's tile of 32 x 32 reads 16 numbers of shared memory for 128 multiply-adds of a lane.
 // (tf32 numbers, of 11 bits, would need three products of half the rate, and their remainders are 2^-22 each.)
 //
 // A number that is not finite has no such sum: its products are NaN. Whoever uses these products looks at the sums and
@@ -19,12 +20,20 @@ namespace split {
 
 // Two neighbouring terms (the first in the lower half), as the operand registers of mma.sync hold them.
 __device__ __forceinline__ void cut(float x0, float x1, uint32_t& h, uint32_t& m, uint32_t& l) {
-  auto upper = [](float a, float b) { return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632); };
-  auto rest = [](float x) { return x - __uint_as_float(__float_as_uint(x) & 0xffff0000u); };
-  h = upper(x0, x1);
-  x0 = rest(x0), x1 = rest(x1);
-  m = upper(x0, x1);
-  l = upper(rest(x0), rest(x1));
+  auto pack = [](float a, float b) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+    return r;
+  };
+  auto rest = [](float& a, float& b, uint32_t r) {
+    a -= __uint_as_float(r << 16);
+    b -= __uint_as_float(r & 0xffff0000u);
+  };
+  h = pack(x0, x1);
+  rest(x0, x1, h);
+  m = pack(x0, x1);
+  rest(x0, x1, m);
+  l = pack(x0, x1);
 }
 
 // Operands of one m16n8k16 product. Lane = 4 g + q. A: terms (0, 1) of row g, of row g + 8, terms (2, 3) of row g, of
@@ -70,6 +79,58 @@ __device__ __forceinline__ void multiply_add(float (&acc)[N][4], const A& a, con
   for (int j = 0; j < N; ++j)
 #pragma unroll
     for (int e = 0; e < 4; ++e) acc[j][e] += t[j][e] + d[j][e];
+}
+
+// The same for accumulators that can afford a second register each: the small products of all terms run on in `low`,
+// 2^-8 of the sum, which is added at the end (one rounding where `multiply_add` has one for every sixteen terms).
+template <int N>
+__device__ __forceinline__ void multiply_add(float (&acc)[N][4], float (&low)[N][4], const A& a, const B (&b)[N]) {
+  float t[N][4];
+#pragma unroll
+  for (int j = 0; j < N; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) t[j][e] = 0.f;
+#pragma unroll
+  for (int j = 0; j < N; ++j) mma(t[j], a.h, b[j].h);
+#pragma unroll
+  for (int j = 0; j < N; ++j) mma(low[j], a.l, b[j].h);
+#pragma unroll
+  for (int j = 0; j < N; ++j) mma(low[j], a.h, b[j].l);
+#pragma unroll
+  for (int j = 0; j < N; ++j) mma(low[j], a.m, b[j].m);
+#pragma unroll
+  for (int j = 0; j < N; ++j) mma(low[j], a.m, b[j].h);
+#pragma unroll
+  for (int j = 0; j < N; ++j) mma(low[j], a.h, b[j].m);
+#pragma unroll
+  for (int j = 0; j < N; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[j][e] += t[j][e];
+}
+// One tile, 16 N terms at a time: acc += a[0] b[0] + .. + a[N - 1] b[N - 1], small products in `low[i]`.
+template <int N>
+__device__ __forceinline__ void multiply_add_terms(float (&acc)[4], float (&low)[N][4], const A (&a)[N], const B (&b)[N]) {
+  float t[N][4];
+#pragma unroll
+  for (int j = 0; j < N; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) t[j][e] = 0.f;
+#pragma unroll
+  for (int j = 0; j < N; ++j) mma(t[j], a[j].h, b[j].h);
+#pragma unroll
+  for (int j = 0; j < N; ++j) mma(low[j], a[j].l, b[j].h);
+#pragma unroll
+  for (int j = 0; j < N; ++j) mma(low[j], a[j].h, b[j].l);
+#pragma unroll
+  for (int j = 0; j < N; ++j) mma(low[j], a[j].m, b[j].m);
+#pragma unroll
+  for (int j = 0; j < N; ++j) mma(low[j], a[j].m, b[j].h);
+#pragma unroll
+  for (int j = 0; j < N; ++j) mma(low[j], a[j].h, b[j].m);
+#pragma unroll
+  for (int j = 0; j < N; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[e] += t[j][e];
 }
 
 // Sixteen terms that lie side by side, rows `ld` apart (16 more than a multiple of 32: no bank conflicts): a lane has

@@ -409,6 +409,32 @@ def test_a_key_is_found_again_in_the_channels_that_kept_it(ops, gap):
     assert out[:2].abs().max() == 0
 
 
+@pytest.mark.parametrize("dk,dv", [(16, 20), (132, 24), (256, 16)])
+@pytest.mark.parametrize("channels", [True, False])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_a_value_that_is_no_number_stays_in_its_column_of_the_state(ops, dk, dv, channels, bad):
+    """The state's columns share products in the chunks; the others keep their bits, the column itself does not recover."""
+    n, col, at = 200, 5, 70
+    qkv = rnd(n, 2 * dk + dv, seed=dk, scale=dk ** -0.5)
+    scal = torch.zeros(n, 1, 4)
+    scal[:, :, 0], scal[:, :, 1] = 1.0 if channels else 0.9, 0.5
+    decay = torch.rand(n, dk, generator=torch.Generator().manual_seed(2)).cuda() if channels else None
+
+    def run(x):
+        S = torch.zeros(1, 1, dv, dk).cuda()
+        out = ops.delta_rule(x.cuda(), scal.cuda(), num_heads=1, num_kv_heads=1, key_dim=dk, value_dim=dv, state=S,
+                             step=batch([n], [0], [0]), decay=decay)
+        return out.cpu(), S[0, 0].cpu()
+
+    out, S = run(qkv)
+    qkv[at, 2 * dk + col] = bad
+    out2, S2 = run(qkv)
+    others = [c for c in range(dv) if c != col]
+    assert torch.equal(out2[:, others], out[:, others]) and torch.equal(S2[others], S[others])
+    assert torch.equal(out2[:64], out[:64])  # the chunk before
+    assert not bool(out2[at:, col].isfinite().any()) and not bool(S2[col].isfinite().any())
+
+
 @pytest.mark.parametrize("dtype", BOTH)
 @pytest.mark.parametrize("T,W,E,top", [(7, 64, 6, 2), (40, 128, 40, 5), (4, 32, 5, 5), (30, 70, 12, 1)])
 def test_router_hands_on_the_scores_as_they_are(ops, dtype, T, W, E, top):
